@@ -604,6 +604,7 @@ hx_status hx_batch_create(hx_batch** out, uint32_t n_maps, const int32_t* size_p
   *out = b;
   hx_status st = hx_batch_clear(b, stream);
   if (st == HX_OK && (e = cudaStreamSynchronize(s)) != cudaSuccess) st = cuda_status(e);
+  pool_object(+1);
   if (st != HX_OK) {
     hx_batch_destroy(b);
     *out = nullptr;
@@ -620,6 +621,7 @@ hx_status hx_batch_destroy(hx_batch* b) {
   cudaFree(b->d_info);
   cudaFree(b->scratch);
   delete b;
+  pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);
 }
 

@@ -669,7 +669,7 @@ static hx_status ensure_scratch(hx_map* m, uint64_t bytes, cudaStream_t s) {
   m->scratch_bytes = 0;
   uint64_t b = 1;
   while (b < bytes) b <<= 1;
-  HX_CUDA(cudaMallocAsync(&m->scratch, b, s));
+  HX_CUDA(pool_alloc(&m->scratch, b, s));
   m->scratch_bytes = b;
   return HX_OK;
 }
@@ -687,7 +687,7 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
   if (new_sp < 1 || new_sp > 31) return HX_ERR_INVALID_ARG;
   const uint64_t nn = 1ull << new_sp;
   void* nt = nullptr;
-  HX_CUDA(cudaMallocAsync(&nt, nn * pair_bytes(m), s));
+  HX_CUDA(pool_alloc(&nt, nn * pair_bytes(m), s));
   hx_status st = fill_empty(m, nt, nn, s);
   if (st != HX_OK) return st;
   k_info_reset<<<1, 1, 0, s>>>(m->info);
@@ -840,6 +840,7 @@ hx_status hx_map_create(hx_map** out, int key_bytes, int val_bytes, int size_pow
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(cuda_status(e));
   *out = m;
+  pool_object(+1);
   return HX_OK;
 }
 
@@ -850,6 +851,7 @@ hx_status hx_map_destroy(hx_map* m) {
   if (m->info) cudaFree(m->info);
   if (m->scratch) cudaFree(m->scratch);
   delete m;
+  pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);
 }
 

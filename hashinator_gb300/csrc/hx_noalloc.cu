@@ -12,8 +12,6 @@
 // from module load until the process exits. All calls share it, so calls
 // that overlap on the GPU corrupt each other's results: order them on one
 // stream (or otherwise serialise them).
-#include <cuda.h>
-
 #include <mutex>
 
 #include "hx_host.h"
@@ -32,33 +30,6 @@ static_assert(hxs::kScratchBytes <= HX_NOALLOC_SCAN_SCRATCH_BYTES, "error word +
 // Scratch of the no-allocation scan, HX_NOALLOC_SCAN_SCRATCH_BYTES
 // (524,544 B): room for either scan kernel's words at n = 2^28.
 static __device__ __align__(256) unsigned char g_noalloc_scan_scratch[HX_NOALLOC_SCAN_SCRATCH_BYTES];
-
-// The current context's driver-assigned id (unique for the life of the
-// process), through the runtime's driver entry points so that libhx does not
-// link libcuda. 0 when the driver does not provide it.
-static unsigned long long current_context_id() {
-  using GetCurrent = CUresult (*)(CUcontext*);
-  using GetId = CUresult (*)(CUcontext, unsigned long long*);
-  static GetCurrent get_current = nullptr;
-  static GetId get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaDriverEntryPointQueryResult q;
-    void* f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<GetCurrent>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<GetId>(f);
-  });
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
-    return 0;
-  return id;
-}
 
 // Device address of the array in the current device's context. In host code
 // the array's name is only a host-side stand-in, so the address comes from

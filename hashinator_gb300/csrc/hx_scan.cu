@@ -1,5 +1,7 @@
 // hx_scan.cu — split::tools replacements (exclusive scan, copy_if) and the
 // host helpers shared by libhx.
+#include <cuda.h>
+
 #include <cstring>
 #include <mutex>
 #include "hx_host.h"
@@ -37,6 +39,83 @@ int sm_count() {
   return cache[dev];
 }
 
+// The current context's driver-assigned id (unique for the life of the
+// process), through the runtime's driver entry points so that libhx does not
+// link libcuda. 0 when the driver does not provide it.
+unsigned long long current_context_id() {
+  using GetCurrent = CUresult (*)(CUcontext*);
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static GetCurrent get_current = nullptr;
+  static GetId get_id = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaDriverEntryPointQueryResult q;
+    void* f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_current = reinterpret_cast<GetCurrent>(f);
+    f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<GetId>(f);
+  });
+  CUcontext ctx = nullptr;
+  unsigned long long id = 0;
+  if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+static std::mutex g_pool_mu;
+static struct {
+  cudaMemPool_t pool;
+  unsigned long long ctx;  // the context that it was created in; a reset device has another one
+} g_pools[64];
+static int g_pool_objects = 0;
+
+cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, s);
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  const unsigned long long ctx = current_context_id();
+  auto& of = g_pools[dev];
+  if (ctx && (!of.pool || of.ctx != ctx)) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return cudaMallocAsync(p, bytes, s);  // nothing but stream work while a capture runs
+    }
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    of.pool = nullptr;
+    cudaMemPool_t made = nullptr;
+    if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
+      uint64_t keep = kPoolKeepBytes;
+      cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+      of.pool = made;
+      of.ctx = ctx;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  if (!ctx || !of.pool) return cudaMallocAsync(p, bytes, s);
+  return cudaMallocFromPoolAsync(p, bytes, of.pool, s);
+}
+
+void pool_object(int change) {
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  g_pool_objects += change;
+  if (change > 0 || g_pool_objects > 0) return;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  const auto& of = g_pools[dev];
+  if (of.pool && of.ctx == current_context_id()) cudaMemPoolTrimTo(of.pool, kPoolIdleBytes);
+}
+
 hx_status Scratch::get(void* caller, uint64_t caller_bytes, uint64_t need, cudaStream_t stream) {
   s = stream;
   if (caller) {
@@ -45,7 +124,7 @@ hx_status Scratch::get(void* caller, uint64_t caller_bytes, uint64_t need, cudaS
     owned = false;
     return HX_OK;
   }
-  HX_CUDA(cudaMallocAsync(&ptr, need, stream));
+  HX_CUDA(pool_alloc(&ptr, need, stream));
   owned = true;
   return HX_OK;
 }
