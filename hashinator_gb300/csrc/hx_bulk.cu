@@ -1,0 +1,250 @@
+// hx_bulk.cu — host side of the slice-by-slice batches (hx_bulk.cuh).
+#include <cmath>
+
+#include "hx_bulk.cuh"
+#include "hx_host.h"
+#include "hx_internal.h"
+
+namespace hx {
+
+// Room of a bin that gets `mean` of the batch's keys on average: eight standard
+// deviations of a random spread above it, so that with keys that hash evenly no
+// bin ever fills.
+static unsigned bulk_bin_room(uint64_t mean) {
+  const double r = (double)mean + 8.0 * std::sqrt((double)mean) + 64.0;
+  return ((unsigned)r + 31u) & ~31u;
+}
+
+static int log2_ceil(uint64_t x) {
+  int l = 0;
+  while ((1ull << l) < x) ++l;
+  return l;
+}
+
+constexpr uint64_t kBulkChunk = 1ull << 27;  // keys of one batch at a time: bounds the scratch
+
+// Scratch of one batch of n records of which `expected` hold keys, in the order
+// [counts][bins of the second split][bins of the first split / left records / found records].
+template <class P, BulkOp OP>
+struct BulkPlan {
+  using K = typename PairTraits<P>::K;
+  using V = typename PairTraits<P>::V;
+  int log1 = 0, log2 = 0;  // digits of the two splits; log1 = 0: one split
+  unsigned room1 = 0, room2 = 0;
+  int region_log = 0;
+  unsigned regions = 0;
+  uint64_t count_words = 0, bin_records = 0, total = 0;
+  uint64_t at_keys2 = 0, at_pay2 = 0, at_keys1 = 0, at_pay1 = 0;
+  static constexpr unsigned kPay = OP == BulkOp::ERASE ? 0 : sizeof(typename BulkPay<P, OP>::T);
+
+  BulkPlan(int sp, uint64_t n, uint64_t expected) {
+    const int bits = sp - slice_log<P>();
+    log2 = bits <= kMaxDigitLog ? bits : bits / 2;
+    log1 = bits - log2;
+    const uint64_t slices = 1ull << bits;
+    room2 = bulk_bin_room(expected >> bits);
+    room1 = log1 ? bulk_bin_room(expected >> log1) : 0;
+    if (OP == BulkOp::FIND) {
+      region_log = log2_ceil(n) - kRegionLog;
+      if (region_log < 10) region_log = 10;
+      regions = (unsigned)((n + (1ull << region_log) - 1) >> region_log);
+    }
+    count_words = slices * 2 + (1ull << log1) + kMaxRegions;  // bins, left, first split, found
+    auto up = [](uint64_t b) { return (b + 255) / 256 * 256; };
+    const uint64_t rec2 = slices * room2, rec1 = (uint64_t)room1 << log1;
+    // the second buffer holds the first split's bins, then the left records of inserts
+    // (as many as the bins may hold) or the values found
+    const uint64_t recb = OP == BulkOp::INSERT && rec2 > rec1 ? rec2 : rec1;
+    uint64_t at = up(count_words * 4);
+    at_keys2 = at;
+    at += up(rec2 * sizeof(K));
+    at_pay2 = at;
+    at += up(rec2 * kPay);
+    at_keys1 = at;
+    uint64_t second;
+    if (OP == BulkOp::FIND) {
+      second = up(rec1 * sizeof(K)) + up(rec1 * kPay);
+      const uint64_t found = up(((uint64_t)regions << region_log) * sizeof(FoundRec<V>));
+      at_pay1 = at + up(rec1 * sizeof(K));
+      if (found > second) second = found;
+    } else {
+      second = up(recb * sizeof(K)) + up(recb * kPay);
+      at_pay1 = at + up(recb * sizeof(K));
+    }
+    total = at + second;
+  }
+};
+
+template <class Kern>
+static cudaError_t allow_smem(Kern kern, size_t smem) {
+  return smem > 32 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                          : cudaSuccess;
+}
+
+template <class P, BulkOp OP, BulkSrc SRC>
+static hx_status launch_split(const BulkArgs<P>& a, const BulkBins& in, const BulkBins& out, unsigned bins_in,
+                              uint64_t records, int shift, int log_digits, cudaStream_t s) {
+  auto kern = k_bulk_split<P, OP, SRC>;
+  const size_t smem = (size_t)bulk_tile<P, OP>() * bulk_record_bytes<P, OP>();
+  HX_CUDA(allow_smem(kern, smem));
+  const unsigned tiles = (unsigned)((records + bulk_tile<P, OP>() - 1) / bulk_tile<P, OP>());
+  kern<<<tiles * bins_in, kBulkThreads, smem, s>>>(a, in, out, tiles, shift, log_digits);
+  return after_launch();
+}
+
+template <class P, BulkOp OP>
+static hx_status bulk_chunk(const BulkArgs<P>& a, BulkSrc src, uint64_t expected, char* scratch, cudaStream_t s) {
+  const BulkPlan<P, OP> pl(a.sp, a.n, expected);
+  const int bits = pl.log1 + pl.log2;
+  const unsigned slices = 1u << bits;
+  unsigned* counts = reinterpret_cast<unsigned*>(scratch);
+  HX_CUDA(cudaMemsetAsync(counts, 0, pl.count_words * 4, s));
+  BulkBins fine{scratch + pl.at_keys2, scratch + pl.at_pay2, counts, pl.room2, bits};
+  // inserts read a bin more than once, so what is left of it goes to the first split's room;
+  // the others write it over the part of the bin that they have read
+  BulkBins left{scratch + (OP == BulkOp::INSERT ? pl.at_keys1 : pl.at_keys2),
+                scratch + (OP == BulkOp::INSERT ? pl.at_pay1 : pl.at_pay2), counts + slices, pl.room2, bits};
+  BulkBins coarse{scratch + pl.at_keys1, scratch + pl.at_pay1, counts + 2ull * slices, pl.room1, pl.log1};
+  unsigned* found = counts + 2ull * slices + (1u << pl.log1);
+  const BulkBins none{};
+  const BulkBins& to = pl.log1 ? coarse : fine;
+  const int shift1 = slice_log<P>() + (pl.log1 ? pl.log2 : 0), digits1 = pl.log1 ? pl.log1 : pl.log2;
+  hx_status st;
+  if (src == BulkSrc::PAIRS) st = launch_split<P, OP, BulkSrc::PAIRS>(a, none, to, 1, a.n, shift1, digits1, s);
+  else if (src == BulkSrc::INDEX && OP == BulkOp::INSERT)
+    st = launch_split<P, OP, OP == BulkOp::INSERT ? BulkSrc::INDEX : BulkSrc::KEYS>(a, none, to, 1, a.n, shift1,
+                                                                                   digits1, s);
+  else st = launch_split<P, OP, BulkSrc::KEYS>(a, none, to, 1, a.n, shift1, digits1, s);
+  if (st != HX_OK) return st;
+  if (pl.log1) {
+    st = launch_split<P, OP, BulkSrc::BINS>(a, coarse, fine, 1u << pl.log1, pl.room1, slice_log<P>(), pl.log2, s);
+    if (st != HX_OK) return st;
+  }
+  auto kern = k_bulk_slice<P, OP>;
+  void* recs = scratch + pl.at_keys1;
+  HX_CUDA(allow_smem(kern, slice_smem<P, OP>()));
+  kern<<<slices, kSliceThreads, slice_smem<P, OP>(), s>>>(a, fine, left, recs, found, pl.region_log);
+  if ((st = after_launch()) != HX_OK) return st;
+  if constexpr (OP == BulkOp::FIND) {
+    const unsigned parts = (unsigned)(((1ull << pl.region_log) + kScatterRecs - 1) / kScatterRecs);
+    k_bulk_scatter<P><<<pl.regions * parts, 256, 0, s>>>(a, recs, found, pl.region_log, parts);
+    if ((st = after_launch()) != HX_OK) return st;
+  }
+  k_bulk_left<P, OP><<<(slices + 7) / 8, 256, 0, s>>>(a, left, slices);
+  return after_launch();
+}
+
+template <class P, BulkOp OP>
+static hx_status bulk_run(BulkArgs<P> a, BulkSrc src, uint64_t expected, cudaStream_t s, bool* done) {
+  *done = false;
+  const uint64_t n = a.n;
+  uint64_t chunk = n < kBulkChunk ? n : kBulkChunk;
+  if (OP == BulkOp::INSERT) {  // a bin's new keys are sorted in shared memory
+    uint64_t mean = bin_room_max<P>();
+    while (bulk_bin_room(mean) > bin_room_max<P>()) mean -= 32;
+    const double share = (double)(mean << (a.sp - slice_log<P>())) / (double)expected;  // of the batch, at once
+    if (share < 1.0) {
+      const uint64_t pieces = (uint64_t)std::ceil(1.0 / share);
+      const uint64_t most = (n + pieces - 1) / pieces;
+      if (chunk > most) chunk = most;
+    }
+  }
+  const uint64_t exp1 = expected < n ? (uint64_t)((double)expected * ((double)chunk / (double)n)) : chunk;
+  const BulkPlan<P, OP> pl(a.sp, chunk, exp1);
+  void* scratch = nullptr;
+  if (pool_alloc(&scratch, pl.total, s) != cudaSuccess) {
+    cudaGetLastError();  // no room for the scratch: the caller probes directly
+    return HX_OK;
+  }
+  hx_status st = HX_OK;
+  const BulkArgs<P> all = a;
+  for (uint64_t at = 0; at < n && st == HX_OK; at += chunk) {
+    a.n = n - at < chunk ? n - at : chunk;
+    a.first = all.first + at;
+    if (all.keys) a.keys = all.keys + at;
+    if (all.vals) a.vals = all.vals + at;
+    if (all.pairs) a.pairs = all.pairs + at;
+    if (all.out) a.out = all.out + at * all.out_stride;
+    st = bulk_chunk<P, OP>(a, src, exp1, static_cast<char*>(scratch), s);
+  }
+  *done = true;
+  HX_CUDA(cudaFreeAsync(scratch, s));
+  return st;
+}
+
+// The rule: a batch goes slice by slice if it has at least one key per `spread`
+// buckets. A slice costs the same however few of its buckets the batch asks for, and
+// probing directly costs more the fuller the table is and, above about 128 MiB, the
+// less of it stays in L2; a look-up costs more here than an insert or an erase (its
+// value has to go back to its place). Measured on GB300, direct time over slice time
+// for u32 / u64 tables of 256-512 MiB:
+//   load factor 0.5:  insert 1/4 1.42 / 1.15, 1/8 1.03 / 0.90; erase 1/4 1.51 / 1.16;
+//                     look-up 1/2 1.18 / 0.90
+//   load factor 0.75: insert 1/8 1.42 / 1.44, 1/16 1.04 / 1.02; erase 1/8 1.46 / 1.76;
+//                     look-up 1/4 1.49 / 1.48, 1/8 1.15 / 1.13
+//   load factor 0.9:  insert 1/16 2.17 / 2.82; erase 4.0 / 5.3; look-up 1.77 / 1.59
+// and for tables of 16-32 MiB, 1/2: at 0.75 1.15 / 1.36, 1.38 / 1.40, 1.18 / 1.35; at
+// 0.9, 1/4: 2.0 / 3.2, 3.1 / 4.5, 1.6 / 1.6. The load factor is the host's bound of it
+// (after the inserts of this call); a bound above the table's size says nothing, and
+// counts as a low one.
+#ifndef HX_BULK_ALWAYS
+#define HX_BULK_ALWAYS 0
+#endif
+static bool bulk_pays(const BulkCall& c) {
+  const uint64_t slots = 1ull << c.sp, bytes = (uint64_t)(c.key_bytes * 2) << c.sp;
+  const int bits = c.sp - (c.key_bytes == 4 ? slice_log<P32>() : slice_log<P64>());
+  if (bits < 1 || bits > 2 * kMaxDigitLog) return false;
+  if (HX_BULK_ALWAYS) return true;
+  const double lf = c.fill_bound <= slots ? (double)c.fill_bound / (double)slots : 0.0;
+  const bool find = c.op == BulkOp::FIND;
+  unsigned spread = 0;
+  if (bytes >= (128ull << 20)) {
+    if (lf >= 0.85) spread = 16;
+    else if (lf >= 0.7) spread = find ? 4 : 8;
+    else spread = !find ? 4 : (c.key_bytes == 4 ? 2 : 0);
+  } else if (bytes >= (16ull << 20)) {
+    if (lf >= 0.85) spread = 4;
+    else if (lf >= 0.7) spread = 2;
+  }
+  return spread && c.expected >= slots / spread;
+}
+
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cs != cudaStreamCaptureStatusNone;
+}
+
+template <class P>
+static hx_status bulk_typed(const BulkCall& c, cudaStream_t s, bool* done) {
+  using K = typename PairTraits<P>::K;
+  using V = typename PairTraits<P>::V;
+  BulkArgs<P> a{};
+  a.table = static_cast<P*>(c.table);
+  a.sp = c.sp;
+  a.info = c.info;
+  a.keys = static_cast<const K*>(c.keys);
+  a.vals = static_cast<const V*>(c.vals);
+  a.pairs = static_cast<const P*>(c.pairs);
+  a.n = c.n;
+  a.out_stride = c.pairs ? 2 : 1;
+  a.out = c.pairs ? reinterpret_cast<V*>(static_cast<P*>(c.out)) + 1 : static_cast<V*>(c.out);
+  const BulkSrc src = c.pairs ? BulkSrc::PAIRS : (c.op == BulkOp::INSERT && !c.vals ? BulkSrc::INDEX : BulkSrc::KEYS);
+  if (c.op != BulkOp::FIND) a.out = nullptr;
+  switch (c.op) {
+    case BulkOp::INSERT: return bulk_run<P, BulkOp::INSERT>(a, src, c.expected, s, done);
+    case BulkOp::FIND: return bulk_run<P, BulkOp::FIND>(a, src, c.expected, s, done);
+    default: return bulk_run<P, BulkOp::ERASE>(a, src, c.expected, s, done);
+  }
+}
+
+hx_status bulk_try(const BulkCall& c, cudaStream_t s, bool* done) {
+  *done = false;
+  if (!bulk_pays(c) || capturing(s)) return HX_OK;
+  return c.key_bytes == 4 ? bulk_typed<P32>(c, s, done) : bulk_typed<P64>(c, s, done);
+}
+
+}  // namespace hx

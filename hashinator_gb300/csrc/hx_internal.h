@@ -43,4 +43,24 @@ hx_status map_find_view(hx_map* m, const void* keys, void* vals, void* pairs, ui
 // device_rehash of the viewed table into a new cudaMallocAsync allocation of
 // 2^new_sp buckets; the old bucket array is released stream-ordered.
 hx_status map_rehash_view(hx_map* m, int new_sp, cudaStream_t s);
+
+// A batch on one table, for the slice-by-slice kernels (hx_bulk.cu).
+enum class BulkOp : int { INSERT, FIND, ERASE };
+struct BulkCall {
+  BulkOp op;
+  int key_bytes;
+  void* table;
+  int sp;
+  DInfo* info;
+  const void* keys;   // keys (with vals: inserts; without: inserts of the index, look-ups, erases) ...
+  const void* vals;
+  const void* pairs;  // ... or pairs; look-ups write pairs' values
+  void* out;          // look-ups: the values, or the pairs
+  uint64_t n;
+  uint64_t expected;  // about how many of the n records hold a key (sentinels are skipped)
+  uint64_t fill_bound;  // the host's bound of the keys in the table after this call's inserts
+};
+// Runs the batch if the rule for such sizes says so and its scratch can be had;
+// *done says whether it did (if not, nothing was launched).
+hx_status bulk_try(const BulkCall& c, cudaStream_t s, bool* done);
 }  // namespace hx

@@ -693,6 +693,17 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
   k_info_reset<<<1, 1, 0, s>>>(m->info);
   if ((st = after_launch()) != HX_OK) return st;
   const uint64_t on = nslots(m);
+  const uint64_t held = m->fill_ub < on ? m->fill_ub : on;
+  bool done = false;
+  st = bulk_try(BulkCall{BulkOp::INSERT, m->key_bytes, nt, new_sp, m->info, nullptr, nullptr, m->buckets, nullptr, on,
+                         held, held}, s, &done);
+  if (st != HX_OK) return st;
+  if (done) {
+    HX_CUDA(cudaFreeAsync(m->buckets, s));
+    m->buckets = nt;
+    m->sp = new_sp;
+    return HX_OK;
+  }
   if (is_p32(m)) {
     auto kern = k_rehash<P32, 4>;
     const bool small = nn < 4;
@@ -733,6 +744,16 @@ static hx_status maybe_grow(hx_map* m, uint64_t n, float target_lf, cudaStream_t
   if (want <= m->sp) return HX_OK;
   if (want > 31) return HX_ERR_INVALID_ARG;
   return rehash(m, (int)want, s);
+}
+
+// Large batches on large tables go slice by slice (hx_bulk.cu), unless the
+// caller has chosen a probe geometry of its own.
+static hx_status try_bulk(const hx_map* m, BulkOp op, const void* keys, const void* vals, const void* pairs, void* out,
+                          uint64_t n, cudaStream_t s, bool* done) {
+  *done = false;
+  if (m->tune.group != 0 || !m->tune.blind || m->tune.wide) return HX_OK;
+  return bulk_try(BulkCall{op, m->key_bytes, m->buckets, m->sp, m->info, keys, vals, pairs, out, n, n, m->fill_ub},
+                  s, done);
 }
 
 static bool valid_map(const hx_map* m) { return m && m->buckets && m->info; }
@@ -868,6 +889,8 @@ hx_status hx_insert(hx_map* m, const void* d_keys, const void* d_vals, uint64_t 
   if (st != HX_OK) return st;
   HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
   m->fill_ub += n;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::INSERT, d_keys, d_vals, nullptr, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, d_keys, d_vals, nullptr, n, nullptr, s)
                    : launch_insert<P64>(m, d_keys, d_vals, nullptr, n, nullptr, s);
 }
@@ -884,6 +907,8 @@ hx_status hx_insert_index(hx_map* m, const void* d_keys, uint64_t n, float targe
   if (st != HX_OK) return st;
   HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
   m->fill_ub += n;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::INSERT, d_keys, nullptr, nullptr, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, d_keys, nullptr, nullptr, n, nullptr, s)
                    : launch_insert<P64>(m, d_keys, nullptr, nullptr, n, nullptr, s);
 }
@@ -900,6 +925,8 @@ hx_status hx_insert_pairs(hx_map* m, const void* d_pairs, uint64_t n, float targ
   if (st != HX_OK) return st;
   HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
   m->fill_ub += n;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::INSERT, nullptr, nullptr, d_pairs, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, nullptr, nullptr, d_pairs, n, nullptr, s)
                    : launch_insert<P64>(m, nullptr, nullptr, d_pairs, n, nullptr, s);
 }
@@ -911,6 +938,9 @@ hx_status hx_retrieve(hx_map* m, const void* d_keys, void* d_vals, uint64_t n, h
   if (!d_keys || !d_vals) return HX_ERR_INVALID_ARG;
   if (misaligned(d_keys, key_bytes(m)) || misaligned(d_vals, key_bytes(m))) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  hx_status st;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::FIND, d_keys, nullptr, nullptr, d_vals, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_find<P32, false>(m, d_keys, d_vals, nullptr, n, s)
                    : launch_find<P64, false>(m, d_keys, d_vals, nullptr, n, s);
 }
@@ -922,6 +952,9 @@ hx_status hx_retrieve_pairs(hx_map* m, void* d_pairs, uint64_t n, hx_stream stre
   if (!d_pairs) return HX_ERR_INVALID_ARG;
   if (misaligned(d_pairs, pair_bytes(m))) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  hx_status st;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::FIND, nullptr, nullptr, d_pairs, d_pairs, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_find<P32, false>(m, nullptr, nullptr, d_pairs, n, s)
                    : launch_find<P64, false>(m, nullptr, nullptr, d_pairs, n, s);
 }
@@ -933,6 +966,9 @@ hx_status hx_erase(hx_map* m, const void* d_keys, uint64_t n, hx_stream stream) 
   if (!d_keys) return HX_ERR_INVALID_ARG;
   if (misaligned(d_keys, key_bytes(m))) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  hx_status st;
+  bool done = false;
+  if ((st = try_bulk(m, BulkOp::ERASE, d_keys, nullptr, nullptr, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_find<P32, true>(m, d_keys, nullptr, nullptr, n, s)
                    : launch_find<P64, true>(m, d_keys, nullptr, nullptr, n, s);
 }

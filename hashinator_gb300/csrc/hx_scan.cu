@@ -103,7 +103,16 @@ cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s) {
     }
   }
   if (!ctx || !of.pool) return cudaMallocAsync(p, bytes, s);
-  return cudaMallocFromPoolAsync(p, bytes, of.pool, s);
+  e = cudaMallocFromPoolAsync(p, bytes, of.pool, s);
+  if (e == cudaSuccess && bytes >= kPoolKeepBytes / 256) {
+    // the threshold counts what is in use too (grown tables): keep kPoolKeepBytes beyond that
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(of.pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
+      used += kPoolKeepBytes;
+      cudaMemPoolSetAttribute(of.pool, cudaMemPoolAttrReleaseThreshold, &used);
+    }
+  }
+  return e;
 }
 
 void pool_object(int change) {
