@@ -343,6 +343,8 @@ __global__ void k_batch_info_reset(DInfo* info, unsigned n) {
     info[i].err = HX_STATUS_SUCCESS;
     info[i].moved = 0;
     info[i].skip = 0;
+    info[i].done = info[i].max_next = 0;
+    info[i].left_next = info[i].moved_next = info[i].left = 0;
   }
 }
 

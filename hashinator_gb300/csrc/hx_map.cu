@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include "hx_clean.cuh"
 #include "hx_host.h"
 #include "hx_internal.h"
 #include "hx_probe.cuh"
@@ -43,19 +44,8 @@ __global__ void k_info_reset(DInfo* info) {
   info->err = HX_STATUS_SUCCESS;
   info->moved = 0;
   info->skip = 0;
-}
-
-// clean_tombstones prologue: nothing to do without tombstones
-// (hashinator.h:1264-1266); else tombstones := 0 and the probe bound restarts
-// from the keys left in their home bucket (hashinator.h:1301).
-__global__ void k_clean_prologue(DInfo* info) {
-  const bool skip = info->tombstones == 0;
-  info->skip = skip ? 1u : 0u;
-  info->moved = 0;
-  if (!skip) {
-    info->tombstones = 0;
-    info->max_probe = info->fill ? 1u : 0u;
-  }
+  info->done = info->max_next = 0;
+  info->left_next = info->moved_next = info->left = 0;
 }
 
 __device__ __forceinline__ void publish_counts(DInfo* info, unsigned ins, unsigned maxd, bool fail, int lane) {
@@ -535,12 +525,10 @@ static hx_status launch_insert(hx_map* m, const void* keys, const void* vals, co
                                const unsigned long long* d_n, cudaStream_t s) {
   using K = typename PairTraits<P>::K;
   using V = typename PairTraits<P>::V;
-  // clean_tombstones re-inserts its moved keys (count on the device) into a
-  // table whose fill bound still counts the erased keys: thread-per-key, and
-  // reading the window before any CAS. A moved key left its home because the
-  // home was taken, and mostly still is, so a blind first CAS at home would
-  // mostly fail: window-first took clean on 2^27 buckets from 0.91 to 0.75 ms
-  // (u32, LF 0.5), 2.05 to 1.62 ms (u32, LF 0.9) and 1.43 to 1.18 ms (u64, LF 0.5).
+  // clean_tombstones inserts the keys that its slices could not take (count on
+  // the device) into a table whose fill bound still counts the erased keys:
+  // thread-per-key, and reading the window before any CAS, as such a key's home
+  // is mostly taken.
   const Policy pol = (d_n && m->tune.group == 0) ? Policy{1, 1} : policy(m, Op::INSERT);
   const bool blind = d_n ? false : m->tune.blind;
   const Geo geo = pick_geo(m, pol.G);
@@ -645,6 +633,33 @@ static hx_status launch_find(hx_map* m, const void* keys, void* vals, void* pair
 #undef HX_LAUNCH_RETRIEVE
   }
   return after_launch();
+}
+
+static hx_status ensure_scratch(hx_map* m, uint64_t bytes, cudaStream_t s);
+
+// clean_tombstones: the pass over the slices, then, if there can be any, the keys
+// that it listed (their count stays on the device).
+template <class P>
+static hx_status launch_clean(hx_map* m, cudaStream_t s) {
+  const uint64_t n = nslots(m);
+  const unsigned slots = (unsigned)(n < clean_slice<P>() ? n : clean_slice<P>());
+  const unsigned grid = (unsigned)(n / slots);
+  P* table = static_cast<P*>(m->buckets);
+  uint64_t cap = 0;
+  hx_status st;
+  if (grid > 1) {
+    cap = m->fill_ub < n ? m->fill_ub : n;  // listed keys <= fill <= fill_ub
+    if ((st = ensure_scratch(m, (cap + 1) * sizeof(P), s)) != HX_OK) return st;
+  }
+  constexpr int PER = 32 / sizeof(P);
+  auto launch = [&](auto kern) -> hx_status {
+    const size_t smem = clean_smem<P>(slots);
+    if (smem > 32 * 1024) HX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, kCleanThreads, smem, s>>>(table, slots, m->sp, m->info, static_cast<P*>(m->scratch), cap);
+    return after_launch();
+  };
+  if ((st = slots >= PER ? launch(k_clean<P, PER>) : launch(k_clean<P, 1>)) != HX_OK || grid == 1) return st;
+  return launch_insert<P>(m, nullptr, nullptr, m->scratch, cap, &m->info->left, s);
 }
 
 template <class P>
@@ -799,18 +814,17 @@ static hx_status extract(hx_map* m, const hx_pred* pred, void* d_out, uint64_t c
   unsigned long long* cnt = d_count ? reinterpret_cast<unsigned long long*>(d_count)
                                     : reinterpret_cast<unsigned long long*>(static_cast<char*>(m->scratch) + sc_bytes);
   cudaError_t e;
-  CleanArgs cl{nullptr, nullptr};
   bool sk = false;
   if (p32) {
     using O = typename std::conditional<KEYS, uint32_t, P32>::type;
-    e = launch_compact<P32, false, O>(static_cast<const P32*>(m->buckets), static_cast<O*>(d_out), n, *pred,
+    e = launch_compact<P32, O>(static_cast<const P32*>(m->buckets), static_cast<O*>(d_out), n, *pred,
                                       TableRef<P32>{static_cast<const P32*>(m->buckets), m->sp}, capacity, cnt,
-                                      m->scratch, cl, s, &sk);
+                                      m->scratch, s, &sk);
   } else {
     using O = typename std::conditional<KEYS, uint64_t, P64>::type;
-    e = launch_compact<P64, false, O>(static_cast<const P64*>(m->buckets), static_cast<O*>(d_out), n, *pred,
+    e = launch_compact<P64, O>(static_cast<const P64*>(m->buckets), static_cast<O*>(d_out), n, *pred,
                                       TableRef<P64>{static_cast<const P64*>(m->buckets), m->sp}, capacity, cnt,
-                                      m->scratch, cl, s, &sk);
+                                      m->scratch, s, &sk);
   }
   if (e != cudaSuccess) return cuda_status(e);
   if ((st = after_launch()) != HX_OK) return st;
@@ -978,35 +992,7 @@ hx_status hx_clean_tombstones(hx_map* m, hx_stream stream) {
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::lock_guard<std::mutex> g(m->mu);
-  const uint64_t n = nslots(m);
-  const bool p32 = is_p32(m);
-  const uint64_t need = p32 ? compact_scratch_need<P32>(n) : compact_scratch_need<P64>(n);
-  const uint64_t sc_bytes = (need + 255) / 256 * 256;
-  const uint64_t cap = m->fill_ub < n ? m->fill_ub : n;  // moved keys <= fill <= fill_ub
-  hx_status st = ensure_scratch(m, sc_bytes + (cap + 1) * pair_bytes(m), s);
-  if (st != HX_OK) return st;
-  void* scan_sc = m->scratch;
-  void* list = static_cast<char*>(m->scratch) + sc_bytes;
-  k_clean_prologue<<<1, 1, 0, s>>>(m->info);
-  if ((st = after_launch()) != HX_OK) return st;
-  hx_pred pr{};
-  pr.op = HX_PRED_NOT_HOME;
-  CleanArgs cl{&m->info->skip, &m->info->fill};
-  cudaError_t e;
-  if (p32) {
-    e = launch_compact<P32, true>(static_cast<const P32*>(m->buckets), static_cast<P32*>(list), n, pr,
-                                  TableRef<P32>{static_cast<const P32*>(m->buckets), m->sp}, cap, &m->info->moved,
-                                  scan_sc, cl, s);
-  } else {
-    e = launch_compact<P64, true>(static_cast<const P64*>(m->buckets), static_cast<P64*>(list), n, pr,
-                                  TableRef<P64>{static_cast<const P64*>(m->buckets), m->sp}, cap, &m->info->moved,
-                                  scan_sc, cl, s);
-  }
-  if (e != cudaSuccess) return cuda_status(e);
-  if ((st = after_launch()) != HX_OK) return st;
-  // Re-insert the moved keys; their count stays on the device.
-  return p32 ? launch_insert<P32>(m, nullptr, nullptr, list, cap, &m->info->moved, s)
-             : launch_insert<P64>(m, nullptr, nullptr, list, cap, &m->info->moved, s);
+  return is_p32(m) ? launch_clean<P32>(m, s) : launch_clean<P64>(m, s);
 }
 
 hx_status hx_extract_pattern(hx_map* m, const hx_pred* pred, void* d_out, uint64_t capacity, uint64_t* d_count,

@@ -33,8 +33,13 @@ struct DInfo {
   unsigned int max_probe;  // exact: largest (distance + 1); 0 for an empty map
   int err;                 // HX_STATUS_*
   unsigned long long moved;  // clean_tombstones: number of keys taken out
-  unsigned int skip;         // clean_tombstones: 1 when there were no tombstones
+  unsigned int skip;         // batched clean_tombstones: 1 when there were no tombstones
+  unsigned int done;         // clean_tombstones: CTAs that are done, 0 between calls; so are the next three
+  unsigned long long left_next;   // keys listed for insertion after the pass
+  unsigned long long moved_next;
+  unsigned int max_next;
   unsigned int pad;
+  unsigned long long left;   // clean_tombstones: keys in its list
 };
 
 enum : int { PR_CONTINUE = 0, PR_INSERTED = 1, PR_UPDATED = 2, PR_FAIL = 3 };

@@ -179,8 +179,8 @@ static hx_status copy_if_t(const void* d_in, void* d_out, uint64_t n, const hx_p
     HX_CUDA(cudaMemsetAsync(sc.ptr, 0, 256, s));
   } else {
     typename ElemOps<T>::Ctx ctx{};
-    cudaError_t e = launch_compact<T, false>(static_cast<const T*>(d_in), static_cast<T*>(d_out), n, pr, ctx,
-                                             capacity, cnt, sc.ptr, CleanArgs{nullptr, nullptr}, s, &sk);
+    cudaError_t e = launch_compact<T>(static_cast<const T*>(d_in), static_cast<T*>(d_out), n, pr, ctx,
+                                             capacity, cnt, sc.ptr, s, &sk);
     if (e != cudaSuccess) return cuda_status(e);
     st = after_launch();
     if (st != HX_OK) return st;

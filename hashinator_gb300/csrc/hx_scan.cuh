@@ -298,7 +298,7 @@ struct ElemOps<P32> : PairOps<P32> {};
 template <>
 struct ElemOps<P64> : PairOps<P64> {};
 
-// The kernel variant for a predicate (CLEAN passes always use the generic one).
+// The kernel variant for a predicate.
 template <class T>
 inline int pred_kind(const hx_pred& p) {
   if (p.op == HX_PRED_MASK_EQ) return PK_MASK_EQ;
@@ -325,21 +325,6 @@ __device__ __forceinline__ O project(const T& x) {
   else return x.first;
 }
 
-// clean_tombstones mode (CLEAN): the input is the bucket array itself. Every
-// TOMBSTONE bucket and every selected (moved) bucket is rewritten to
-// (EMPTY, 0) after it has been read, the last tile takes the moved count off
-// fill, and the whole pass is skipped when *skip is set. The
-// phase-partitioned kernel decides "not home" from the bucket's index
-// (home(Y) != i) and reads no other bucket. The look-back kernel reads the
-// home bucket; one that another CTA rewrites at the same time cannot change
-// its decision: a key Y is "not home" iff bucket[home(Y)] holds a key other
-// than Y, and that bucket only ever changes between keys other than Y and
-// EMPTY.
-struct CleanArgs {
-  const unsigned* skip;
-  unsigned long long* fill;
-};
-
 template <class T, int R>
 __device__ __forceinline__ void compact_load(const T* in, uint64_t n, uint64_t chunk, int lane, bool vec,
                                              T (&x)[R][16 / sizeof(T)]) {
@@ -364,11 +349,11 @@ __device__ __forceinline__ void compact_load(const T* in, uint64_t n, uint64_t c
 // output with coalesced stores. Registers hold two sub-tiles whatever S is,
 // and the look-back, which bounds how many tiles per second the GPU can
 // retire, is paid once per S sub-tiles.
-template <class T, class O, int BLOCK, int R, int S, bool CLEAN, int PK>
+template <class T, class O, int BLOCK, int R, int S, int PK>
 __global__ void __launch_bounds__(BLOCK) k_compact(const T* __restrict__ in, O* __restrict__ out, uint64_t n,
                                                   hx_pred pr, uint64_t magic, typename ElemOps<T>::Ctx ctx,
                                                   uint64_t capacity, unsigned long long* d_count, ScanScratch sc,
-                                                  bool vec, CleanArgs cl) {
+                                                  bool vec) {
   constexpr int E = ElemOps<T>::E;
   constexpr int WARPS = BLOCK / 32;
   constexpr uint64_t SUB = (uint64_t)BLOCK * R * E;
@@ -380,9 +365,6 @@ __global__ void __launch_bounds__(BLOCK) k_compact(const T* __restrict__ in, O* 
   O* s_out = reinterpret_cast<O*>(s_raw);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (CLEAN) {
-    if (*cl.skip) return;
-  }
   if (threadIdx.x == 0) s_tile = atomicAdd(sc.ticket, 1u);
   __syncthreads();
   const unsigned long long tile = s_tile;
@@ -405,17 +387,6 @@ __global__ void __launch_bounds__(BLOCK) k_compact(const T* __restrict__ in, O* 
       for (int q = 0; q < E; ++q)
         if (e + q < n && ElemOps<T>::template pred<PK>(pr, x[r][q], ctx, magic)) bits |= 1u << q;
       f[r] = bits;
-      if constexpr (CLEAN) {
-        using Tr = PairTraits<T>;
-#pragma unroll
-        for (int q = 0; q < E; ++q)
-          if (e + q < n && ((bits >> q) & 1u || x[r][q].first == Tr::TOMB)) {
-            T empty;
-            empty.first = Tr::EMPTY;
-            empty.second = 0;
-            const_cast<T*>(in)[e + q] = empty;
-          }
-      }
     }
     unsigned pre[R];
     unsigned acc = 0;
@@ -458,7 +429,6 @@ __global__ void __launch_bounds__(BLOCK) k_compact(const T* __restrict__ in, O* 
       s_prefix = tp;
       if (tile0 + TILE >= n) {  // last tile
         if (d_count) *d_count = tp + staged;
-        if constexpr (CLEAN) atomicAdd(cl.fill, 0ull - (tp + staged));
       }
     }
   }
@@ -559,16 +529,13 @@ inline cudaError_t launch_scan(const uint32_t* in, uint32_t* out, uint64_t n, vo
 }
 
 // The predicate of a compaction for the phase-partitioned kernel: one
-// compiled predicate kind (PK_*), and in clean_tombstones mode (CLEAN) the
-// rewrite of every TOMBSTONE and every selected bucket to (EMPTY, 0) after
-// it has been read (see CleanArgs).
-template <class T, int PK, bool CLEAN>
+// compiled predicate kind (PK_*).
+template <class T, int PK>
 struct PredSel {
   hx_pred pr;
   uint64_t magic;
   typename ElemOps<T>::Ctx ctx;
   uint64_t thresh = 0;  // PK_MOD_LT_THRESH: floor(s * magic / 2^32)
-  static constexpr bool kRewrites = CLEAN;
   // generic pair rules may be HX_PRED_NOT_HOME, which compares a bucket's
   // index with its key's home bucket
   static constexpr bool kIndexed = PK == PK_GENERIC && !std::is_same<T, uint32_t>::value;
@@ -592,51 +559,36 @@ struct PredSel {
       return ElemOps<T>::template pred<PK>(pr, x, ctx, magic);
     }
   }
-  __device__ __forceinline__ void rewrite(T* in, uint64_t i, const T& x, bool selected) const {
-    if constexpr (CLEAN) {
-      using Tr = PairTraits<T>;
-      if (selected || x.first == Tr::TOMB) {
-        T empty;
-        empty.first = Tr::EMPTY;
-        empty.second = 0;
-        in[i] = empty;
-      }
-    }
-  }
 };
 
 // Launch one compaction pass (n > 0) with scratch of compact_scratch_need<T>(n)
 // bytes, which is zeroed here: the phase-partitioned kernel when the input
 // is 16-byte aligned, else the look-back kernel k_compact.
-template <class T, bool CLEAN, class O = T>
+template <class T, class O = T>
 inline cudaError_t launch_compact(const T* in, O* out, uint64_t n, const hx_pred& pr,
                                   typename ElemOps<T>::Ctx ctx, uint64_t capacity, unsigned long long* d_count,
-                                  void* scratch, CleanArgs cl, cudaStream_t s, bool* stream_kernel = nullptr) {
+                                  void* scratch, cudaStream_t s, bool* stream_kernel = nullptr) {
   const bool sk = aligned16(in);
   if (stream_kernel) *stream_kernel = sk;
   if (sk) {
-    const hxs::Done done{d_count, CLEAN ? cl.fill : nullptr, CLEAN ? cl.skip : nullptr};
+    const hxs::Done done{d_count};
     auto go = [&](auto sel) -> cudaError_t {
       return hxs::launch<T, O, decltype(sel), false>(in, out, n, sel, capacity, done, scratch, s);
     };
-    if constexpr (CLEAN) {
-      return go(PredSel<T, PK_GENERIC, true>{pr, 0, ctx});
-    } else {
-      switch (pred_kind<T>(pr)) {
-        case PK_MOD_LT32:
-          if (mod_lt_thresh_ok(pr.a, pr.b)) {
-            const uint64_t m = fastmod_magic((uint32_t)pr.a);
-            return go(PredSel<T, PK_MOD_LT_THRESH, false>{pr, m, ctx, (pr.b * m) >> 32});
-          }
-          return go(PredSel<T, PK_MOD_LT32, false>{pr, fastmod_magic((uint32_t)pr.a), ctx});
-        case PK_MASK_EQ:
-          return go(PredSel<T, PK_MASK_EQ, false>{pr, 0, ctx});
-        case PK_VALID:
-          if constexpr (!std::is_same<T, uint32_t>::value) return go(PredSel<T, PK_VALID, false>{pr, 0, ctx});
-          [[fallthrough]];
-        default:
-          return go(PredSel<T, PK_GENERIC, false>{pr, 0, ctx});
-      }
+    switch (pred_kind<T>(pr)) {
+      case PK_MOD_LT32:
+        if (mod_lt_thresh_ok(pr.a, pr.b)) {
+          const uint64_t m = fastmod_magic((uint32_t)pr.a);
+          return go(PredSel<T, PK_MOD_LT_THRESH>{pr, m, ctx, (pr.b * m) >> 32});
+        }
+        return go(PredSel<T, PK_MOD_LT32>{pr, fastmod_magic((uint32_t)pr.a), ctx});
+      case PK_MASK_EQ:
+        return go(PredSel<T, PK_MASK_EQ>{pr, 0, ctx});
+      case PK_VALID:
+        if constexpr (!std::is_same<T, uint32_t>::value) return go(PredSel<T, PK_VALID>{pr, 0, ctx});
+        [[fallthrough]];
+      default:
+        return go(PredSel<T, PK_GENERIC>{pr, 0, ctx});
     }
   }
   const uint64_t tiles = compact_tiles<T>(n);
@@ -648,25 +600,20 @@ inline cudaError_t launch_compact(const T* in, O* out, uint64_t n, const hx_pred
   auto launch = [&](auto kern, uint64_t magic) -> cudaError_t {
     cudaError_t err = allow_dynamic_smem(kern, smem);
     if (err != cudaSuccess) return err;
-    kern<<<grid, kCompactBlock, smem, s>>>(in, out, n, pr, magic, ctx, capacity, d_count, sc, false, cl);
+    kern<<<grid, kCompactBlock, smem, s>>>(in, out, n, pr, magic, ctx, capacity, d_count, sc, false);
     return cudaGetLastError();
   };
-  if constexpr (CLEAN) {
-    return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, true, PK_GENERIC>, 0);
-  } else {
-    switch (pred_kind<T>(pr)) {
-      case PK_MOD_LT32:
-        return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, false, PK_MOD_LT32>,
-                      fastmod_magic((uint32_t)pr.a));
-      case PK_MASK_EQ:
-        return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, false, PK_MASK_EQ>, 0);
-      case PK_VALID:
-        if constexpr (!std::is_same<T, uint32_t>::value)
-          return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, false, PK_VALID>, 0);
-        [[fallthrough]];
-      default:
-        return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, false, PK_GENERIC>, 0);
-    }
+  switch (pred_kind<T>(pr)) {
+    case PK_MOD_LT32:
+      return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, PK_MOD_LT32>, fastmod_magic((uint32_t)pr.a));
+    case PK_MASK_EQ:
+      return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, PK_MASK_EQ>, 0);
+    case PK_VALID:
+      if constexpr (!std::is_same<T, uint32_t>::value)
+        return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, PK_VALID>, 0);
+      [[fallthrough]];
+    default:
+      return launch(k_compact<T, O, kCompactBlock, kCompactR, kCompactS, PK_GENERIC>, 0);
   }
 }
 

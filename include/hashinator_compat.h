@@ -534,7 +534,6 @@ struct KeyOf {
 template <typename Rule>
 struct RuleSel {
   Rule rule;
-  static constexpr bool kRewrites = false;
   static constexpr bool kIndexed = false;
   template <class T>
   __device__ __forceinline__ bool operator()(const T& x) const {
@@ -542,8 +541,6 @@ struct RuleSel {
     T y = x;
     return r(y);
   }
-  template <class T>
-  __device__ __forceinline__ void rewrite(T*, uint64_t, const T&, bool) const {}
 };
 
 // The first elements of an input that does not start on a 16-byte boundary
@@ -677,7 +674,7 @@ void compact(const T* in, O* out, size_t n, size_t cap, Rule rule, Proj proj, si
       hxcompat::check_cuda(cudaGetLastError(), "k_head");
     }
     if (n > h) {
-      hxs::Done done{cnt, nullptr, nullptr};
+      hxs::Done done{cnt};
       done.count_max = count_max;
       done.base_from = h ? head : nullptr;
       hxcompat::check_cuda(hxs::launch<T, O, RuleSel<Rule>, false>(in + h, out, n - h, RuleSel<Rule>{rule}, cap,
@@ -858,7 +855,7 @@ void compact_loop(SplitVector<T, A>& in, SplitVector<U, B>& out, Rule rule, Proj
     }
     void* sc = nullptr;
     hxcompat::check_cuda(cudaMallocAsync(&sc, compaction_scratch_bytes<T>(nmax), s), "cudaMallocAsync");
-    hxs::Done done{reinterpret_cast<unsigned long long*>(out.size_word()), nullptr, nullptr};
+    hxs::Done done{reinterpret_cast<unsigned long long*>(out.size_word())};
     done.count_max = out.capacity();
     done.n_from = reinterpret_cast<const unsigned long long*>(in.size_word());
     hxcompat::check_cuda(hxs::launch<T, U, RuleSel<Rule>, false>(in.data(), out.data(), nmax, RuleSel<Rule>{rule},

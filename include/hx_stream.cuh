@@ -1,5 +1,5 @@
 // hx_stream.cuh — phase-partitioned streaming kernels: stable stream
-// compaction (copy_if, extractPattern, the clean_tombstones pass) and the
+// compaction (copy_if, extractPattern) and the
 // exclusive u32 scan, for 16-byte-aligned inputs.
 //
 // Header-only so that the drop-in C++ header can instantiate the same
@@ -175,38 +175,27 @@ __device__ __forceinline__ O project(const T& x) {
 
 // Selector concept (compaction): a copyable struct with
 //   __device__ bool operator()(const T& x) const;
-//   static constexpr bool kRewrites;   // true: called as below for every element of the input
-//   __device__ void rewrite(T* in, uint64_t i, const T& x, bool selected) const;
 //   static constexpr bool kIndexed;    // true: the rule is called as at(x, i), i the element's index
-// kRewrites lets the clean_tombstones pass empty the buckets it takes out;
 // kIndexed lets a rule depend on where the element sits (a bucket's home).
 template <class F>
 struct FunctorSel {
   F f;
-  static constexpr bool kRewrites = false;
   static constexpr bool kIndexed = false;
   template <class T>
   __device__ __forceinline__ bool operator()(const T& x) const {
     return f(x);
   }
-  template <class T>
-  __device__ __forceinline__ void rewrite(T*, uint64_t, const T&, bool) const {}
 };
 struct ScanSel {  // placeholder selector of the scan
-  static constexpr bool kRewrites = false;
   static constexpr bool kIndexed = false;
   template <class T>
   __device__ __forceinline__ bool operator()(const T&) const {
     return true;
   }
-  template <class T>
-  __device__ __forceinline__ void rewrite(T*, uint64_t, const T&, bool) const {}
 };
 
 struct Done {                              // what the pass reports, and where it starts
   unsigned long long* d_count;              // if set, *d_count = min(total, count_max) (compaction)
-  unsigned long long* sub_from;             // if set, *sub_from -= total (clean_tombstones' fill)
-  const unsigned* skip;                     // if set and *skip != 0, the pass does nothing at all
   unsigned long long count_max = ~0ull;     // the largest count written to *d_count
   const unsigned long long* base_from = nullptr;  // if set, output starts at out[*base_from] (and
                                                   // the total counts it), after elements placed earlier
@@ -237,7 +226,6 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
 
   // Device-side inputs: the same values for every CTA, so every CTA runs the
   // same phases and none waits on a CTA that skipped.
-  if (done.skip && *done.skip) return;
   if (done.n_from && *done.n_from < n) n = *done.n_from;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned G = gridDim.x, b = blockIdx.x;
@@ -353,7 +341,6 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
               if constexpr (Sel::kIndexed) s = sel.at(x[r][q], e + q);
               else s = sel(x[r][q]);
               m |= (unsigned)s << q;
-              if constexpr (Sel::kRewrites) sel.rewrite(const_cast<T*>(in), e + q, x[r][q], s);
             }
           } else {
 #pragma unroll
@@ -365,9 +352,6 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
                 else s = sel(x[r][q]);
               }
               if (s) m |= 1u << q;
-              if constexpr (Sel::kRewrites) {
-                if (in_range) sel.rewrite(const_cast<T*>(in), e + q, x[r][q], s);
-              }
             }
           }
           bits[r] = m;
@@ -553,7 +537,6 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
   }
   if (b == 0 && threadIdx.x == 0) {
     if (done.d_count) *done.d_count = base < done.count_max ? base : done.count_max;
-    if (done.sub_from) atomicAdd(done.sub_from, 0ull - base);
   }
 }
 
