@@ -348,6 +348,16 @@ __host__ __device__ constexpr unsigned slice_smem() {
          (OP == BulkOp::FIND ? ((1u << slice_log<P>()) + kTailNodes) * sizeof(K) : 0) +
          (OP == BulkOp::INSERT ? bin_room_max<P>() * 2 : 0);
 }
+// Starts bringing `bytes` (a multiple of 16, from a 16-byte boundary) into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
+  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// How many slices ahead a CTA fetches into L2: its first loads then wait for L2 and not
+// for DRAM. 2^27 u32 buckets, 2^26 keys, insert / look-up: 1.34 / 1.60 ms without, 1.24 /
+// 1.51 ms with 228 or 456 slices (half of or all that run at once), 1.28 / 1.53 with 912.
+#ifndef HX_SLICE_AHEAD
+#define HX_SLICE_AHEAD 228
+#endif
 __device__ __forceinline__ uint32_t smem_cas(uint32_t* p, uint32_t e, uint32_t d) { return atomicCAS(p, e, d); }
 __device__ __forceinline__ uint64_t smem_cas(uint64_t* p, uint64_t e, uint64_t d) {
   return atomicCAS(reinterpret_cast<unsigned long long*>(p), (unsigned long long)e, (unsigned long long)d);
@@ -405,6 +415,14 @@ __global__ void __launch_bounds__(kSliceThreads, HX_SLICE_MINB) k_bulk_slice(Bul
     }
   };
 
+  if (tid == 64 && s + HX_SLICE_AHEAD < gridDim.x) {
+    const unsigned f = s + HX_SLICE_AHEAD;
+    prefetch_l2(a.table + ((uint64_t)f << slice_log<P>()), SB * sizeof(P));
+    const unsigned n = min(bins.count[f], bins.room);
+    prefetch_l2(static_cast<const K*>(bins.keys) + (uint64_t)f * bins.room, (n * (unsigned)sizeof(K) + 15) & ~15u);
+    if constexpr (HAS_PAY)
+      prefetch_l2(static_cast<const Y*>(bins.pay) + (uint64_t)f * bins.room, (n * (unsigned)sizeof(Y) + 15) & ~15u);
+  }
   // ---- the slice's keys, those away from home chained ------------------------
   K tk[N][PER];
   V tv[N][PER];
