@@ -209,7 +209,7 @@ static bool bulk_pays(const BulkCall& c) {
   return spread && c.expected >= slots / spread;
 }
 
-static bool capturing(cudaStream_t s) {
+bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
     cudaGetLastError();

@@ -30,6 +30,8 @@ struct hx_map {
   void* scratch = nullptr;
   uint64_t scratch_bytes = 0;
   hx::Tuning tune;
+  bool err_success = false;  // info->err is known to be success (see set_err_success)
+  bool viewed = false;       // a device view was handed out: kernels of the caller may write info->err
   std::mutex mu;  // guards scratch growth; a map is not thread-safe otherwise
 };
 
@@ -60,6 +62,8 @@ struct BulkCall {
   uint64_t expected;  // about how many of the n records hold a key (sentinels are skipped)
   uint64_t fill_bound;  // the host's bound of the keys in the table after this call's inserts
 };
+// Whether the stream is being captured (also if the runtime cannot say).
+bool capturing(cudaStream_t s);
 // Runs the batch if the rule for such sizes says so and its scratch can be had;
 // *done says whether it did (if not, nothing was launched).
 hx_status bulk_try(const BulkCall& c, cudaStream_t s, bool* done);

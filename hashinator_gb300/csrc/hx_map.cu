@@ -22,9 +22,21 @@ namespace hx {
 // kernels
 // ---------------------------------------------------------------------------
 
-// Every bucket := (EMPTY, 0), 16 bytes per store.
+__device__ __forceinline__ void info_reset(DInfo* info) {
+  info->fill = 0;
+  info->tombstones = 0;
+  info->max_probe = 0;
+  info->err = HX_STATUS_SUCCESS;
+  info->moved = 0;
+  info->skip = 0;
+  info->done = info->max_next = 0;
+  info->left_next = info->moved_next = info->left = 0;
+}
+
+// Every bucket := (EMPTY, 0), 16 bytes per store, and the metadata of an empty table.
 template <class P>
-__global__ void k_fill_empty(P* __restrict__ t, uint64_t nslots) {
+__global__ void k_fill_empty(P* __restrict__ t, uint64_t nslots, DInfo* info) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) info_reset(info);
   constexpr int PER = 16 / sizeof(P);
   const uint64_t n16 = nslots / PER;
   uint4 v;
@@ -35,17 +47,6 @@ __global__ void k_fill_empty(P* __restrict__ t, uint64_t nslots) {
     __stcs(p + i, v);
   // odd tail (nslots == 1 for an 8-byte pair table of size power 0 never
   // occurs: size power >= 1)
-}
-
-__global__ void k_info_reset(DInfo* info) {
-  info->fill = 0;
-  info->tombstones = 0;
-  info->max_probe = 0;
-  info->err = HX_STATUS_SUCCESS;
-  info->moved = 0;
-  info->skip = 0;
-  info->done = info->max_next = 0;
-  info->left_next = info->moved_next = info->left = 0;
 }
 
 __device__ __forceinline__ void publish_counts(DInfo* info, unsigned ins, unsigned maxd, bool fail, int lane) {
@@ -467,6 +468,7 @@ static Geo pick_geo(const hx_map* m, int G) {
 template <class F>
 static unsigned grid_for(F kernel, uint64_t work_threads, int block) {
   const uint64_t want = (work_threads + block - 1) / block;
+  if (want <= (uint64_t)sm_count()) return (unsigned)(want ? want : 1);  // no query: one block per SM always fits
   const uint64_t cap = (uint64_t)sm_count() * blocks_per_sm(kernel, block);
   const uint64_t g = want < cap ? want : cap;
   return (unsigned)(g ? g : 1);
@@ -663,10 +665,10 @@ static hx_status launch_clean(hx_map* m, cudaStream_t s) {
 }
 
 template <class P>
-static hx_status launch_fill_empty(void* t, uint64_t n, cudaStream_t s) {
+static hx_status launch_fill_empty(void* t, uint64_t n, DInfo* info, cudaStream_t s) {
   auto kern = k_fill_empty<P>;
   const uint64_t n16 = n * sizeof(P) / 16;
-  kern<<<grid_for(kern, n16, 256), 256, 0, s>>>(static_cast<P*>(t), n);
+  kern<<<grid_for(kern, n16, 256), 256, 0, s>>>(static_cast<P*>(t), n, info);
   return after_launch();
 }
 
@@ -674,7 +676,7 @@ static hx_status fill_empty(hx_map* m, void* t, uint64_t n, cudaStream_t s) {
   if (n * pair_bytes(m) < 16) {  // a 2-bucket u32 table: 16 B, always >= 16
     return HX_ERR_INVALID_ARG;
   }
-  return is_p32(m) ? launch_fill_empty<P32>(t, n, s) : launch_fill_empty<P64>(t, n, s);
+  return is_p32(m) ? launch_fill_empty<P32>(t, n, m->info, s) : launch_fill_empty<P64>(t, n, m->info, s);
 }
 
 static hx_status ensure_scratch(hx_map* m, uint64_t bytes, cudaStream_t s) {
@@ -705,8 +707,6 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
   HX_CUDA(pool_alloc(&nt, nn * pair_bytes(m), s));
   hx_status st = fill_empty(m, nt, nn, s);
   if (st != HX_OK) return st;
-  k_info_reset<<<1, 1, 0, s>>>(m->info);
-  if ((st = after_launch()) != HX_OK) return st;
   const uint64_t on = nslots(m);
   const uint64_t held = m->fill_ub < on ? m->fill_ub : on;
   bool done = false;
@@ -769,6 +769,16 @@ static hx_status try_bulk(const hx_map* m, BulkOp op, const void* keys, const vo
   if (m->tune.group != 0 || !m->tune.blind || m->tune.wide) return HX_OK;
   return bulk_try(BulkCall{op, m->key_bytes, m->buckets, m->sp, m->info, keys, vals, pairs, out, n, n, m->fill_ub},
                   s, done);
+}
+
+// err = success before an insert (hashers.h:50), unless the device word is known to
+// hold it: after a clear, until a kernel that may set fail, a peek_status or a device
+// view (whose kernels write it unseen). A call under capture writes it always, as its
+// replays follow other work than the capture did.
+static hx_status set_err_success(hx_map* m, cudaStream_t s) {
+  if (m->err_success && !capturing(s)) return HX_OK;
+  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
+  return HX_OK;
 }
 
 static bool valid_map(const hx_map* m) { return m && m->buckets && m->info; }
@@ -866,8 +876,6 @@ hx_status hx_map_create(hx_map** out, int key_bytes, int val_bytes, int size_pow
   if (e != cudaSuccess) return fail(cuda_status(e));
   hx_status st = fill_empty(m, m->buckets, nslots(m), s);
   if (st != HX_OK) return fail(st);
-  k_info_reset<<<1, 1, 0, s>>>(m->info);
-  if ((st = after_launch()) != HX_OK) return fail(st);
   // A fresh map reports status::invalid until its first insert
   // (Info(int) constructor, defaults.h:47-49).
   int inv = HX_STATUS_INVALID;
@@ -895,14 +903,13 @@ hx_status hx_insert(hx_map* m, const void* d_keys, const void* d_vals, uint64_t 
   HX_RANGE("hx_insert");
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));  // err = success (hashers.h:50)
-  if (n == 0) return HX_OK;
+  hx_status st = set_err_success(m, s);
+  if (st != HX_OK || n == 0) return st;
   if (!d_keys || !d_vals) return HX_ERR_INVALID_ARG;
   if (misaligned(d_keys, key_bytes(m)) || misaligned(d_vals, key_bytes(m))) return HX_ERR_INVALID_ARG;
-  hx_status st = maybe_grow(m, n, target_lf, s);
-  if (st != HX_OK) return st;
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
+  if ((st = maybe_grow(m, n, target_lf, s)) != HX_OK) return st;
   m->fill_ub += n;
+  m->err_success = false;  // the kernel may set fail
   bool done = false;
   if ((st = try_bulk(m, BulkOp::INSERT, d_keys, d_vals, nullptr, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, d_keys, d_vals, nullptr, n, nullptr, s)
@@ -913,14 +920,13 @@ hx_status hx_insert_index(hx_map* m, const void* d_keys, uint64_t n, float targe
   HX_RANGE("hx_insert_index");
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
-  if (n == 0) return HX_OK;
+  hx_status st = set_err_success(m, s);
+  if (st != HX_OK || n == 0) return st;
   if (!d_keys) return HX_ERR_INVALID_ARG;
   if (misaligned(d_keys, key_bytes(m))) return HX_ERR_INVALID_ARG;
-  hx_status st = maybe_grow(m, n, target_lf, s);
-  if (st != HX_OK) return st;
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
+  if ((st = maybe_grow(m, n, target_lf, s)) != HX_OK) return st;
   m->fill_ub += n;
+  m->err_success = false;
   bool done = false;
   if ((st = try_bulk(m, BulkOp::INSERT, d_keys, nullptr, nullptr, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, d_keys, nullptr, nullptr, n, nullptr, s)
@@ -931,14 +937,13 @@ hx_status hx_insert_pairs(hx_map* m, const void* d_pairs, uint64_t n, float targ
   HX_RANGE("hx_insert_pairs");
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
-  if (n == 0) return HX_OK;
+  hx_status st = set_err_success(m, s);
+  if (st != HX_OK || n == 0) return st;
   if (!d_pairs) return HX_ERR_INVALID_ARG;
   if (misaligned(d_pairs, pair_bytes(m))) return HX_ERR_INVALID_ARG;
-  hx_status st = maybe_grow(m, n, target_lf, s);
-  if (st != HX_OK) return st;
-  HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
+  if ((st = maybe_grow(m, n, target_lf, s)) != HX_OK) return st;
   m->fill_ub += n;
+  m->err_success = false;
   bool done = false;
   if ((st = try_bulk(m, BulkOp::INSERT, nullptr, nullptr, d_pairs, nullptr, n, s, &done)) != HX_OK || done) return st;
   return is_p32(m) ? launch_insert<P32>(m, nullptr, nullptr, d_pairs, n, nullptr, s)
@@ -1019,9 +1024,9 @@ hx_status hx_clear(hx_map* m, hx_stream stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   hx_status st = fill_empty(m, m->buckets, nslots(m), s);
   if (st != HX_OK) return st;
-  k_info_reset<<<1, 1, 0, s>>>(m->info);
   m->fill_ub = 0;
-  return after_launch();
+  m->err_success = !m->viewed && !capturing(s);
+  return HX_OK;
 }
 
 hx_status hx_resize_to_lf(hx_map* m, float target_lf, hx_stream stream) {
@@ -1079,6 +1084,7 @@ hx_status hx_get_info(hx_map* m, hx_info* out, hx_stream stream) {
 hx_status hx_peek_status(hx_map* m, int32_t* out, hx_stream stream) {
   if (!valid_map(m) || !out) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  m->err_success = false;
   int v = 0, inv = HX_STATUS_INVALID;
   HX_CUDA(cudaMemcpyAsync(&v, &m->info->err, sizeof(int), cudaMemcpyDeviceToHost, s));
   HX_CUDA(cudaMemcpyAsync(&m->info->err, &inv, sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1097,6 +1103,8 @@ hx_status hx_map_device_view(hx_map* m, hx_device_view* out) {
   out->max_probe = &m->info->max_probe;
   out->err = &m->info->err;
   m->fill_ub = nslots(m);  // device-side inserts are invisible to the host bound
+  m->viewed = true;
+  m->err_success = false;
   return HX_OK;
 }
 
