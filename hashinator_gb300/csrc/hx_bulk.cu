@@ -174,38 +174,46 @@ static hx_status bulk_run(BulkArgs<P> a, BulkSrc src, uint64_t expected, cudaStr
 
 // The rule: a batch goes slice by slice if it has at least one key per `spread`
 // buckets. A slice costs the same however few of its buckets the batch asks for, and
-// probing directly costs more the fuller the table is and, above about 128 MiB, the
-// less of it stays in L2; a look-up costs more here than an insert or an erase (its
-// value has to go back to its place). Measured on GB300, direct time over slice time
-// for u32 / u64 tables of 256-512 MiB:
-//   load factor 0.5:  insert 1/4 1.42 / 1.15, 1/8 1.03 / 0.90; erase 1/4 1.51 / 1.16;
-//                     look-up 1/2 1.18 / 0.90
-//   load factor 0.75: insert 1/8 1.42 / 1.44, 1/16 1.04 / 1.02; erase 1/8 1.46 / 1.76;
-//                     look-up 1/4 1.49 / 1.48, 1/8 1.15 / 1.13
-//   load factor 0.9:  insert 1/16 2.17 / 2.82; erase 4.0 / 5.3; look-up 1.77 / 1.59
-// and for tables of 16-32 MiB, 1/2: at 0.75 1.15 / 1.36, 1.38 / 1.40, 1.18 / 1.35; at
-// 0.9, 1/4: 2.0 / 3.2, 3.1 / 4.5, 1.6 / 1.6. The load factor is the host's bound of it
-// (after the inserts of this call); a bound above the table's size says nothing, and
-// counts as a low one.
-#ifndef HX_BULK_ALWAYS
-#define HX_BULK_ALWAYS 0
-#endif
+// probing directly costs more the fuller the table is and the less of it stays in L2
+// (128 MiB of it do); a look-up costs more here than an insert or an erase, as its
+// value has to go back to its place. Measured on GB300, direct time over slice time
+// for u32 / u64 tables (of the size in brackets, for one key per so many buckets):
+//   load factor 0.5:  insert [128 MiB] 1/2 1.28 / 1.22, [256] 1/4 1.49 / 1.13; erase
+//                     [256] 1/4 1.5 / 1.2; look-up [256] 1/2 0.92 / 0.86, [1 GiB] 1/2
+//                     1.40 / 1.00, [2 GiB] 1.16 (u64)
+//   load factor 0.72: insert [128] 1/5 0.86 / 0.73, [256] 1/5 1.34 / 1.18; erase [256]
+//                     1/18 1.20 / 1.04; look-up [256] 1/3 0.92 / 0.94, [512] 1.31 (u64)
+//   load factor 0.8:  look-up [256] 1/3 1.20 / 1.3
+//   load factor 0.86: insert [128] 1/5 1.20 / 1.46, [32] 1/5 1.08 / 1.85; erase [128]
+//                     1/15 1.34 / 1.62; look-up [128] 1/5 1.0 / 1.34, [256] 1/5 1.45 / 2.4
+//   load factor 0.92: insert [32] 1/4 2.0 / 4.1; erase [32] 1/14 2.8 / 5.4; look-up
+//                     [32] 1/4 2.1 / 2.2, [128] 2.2 / 3.3
+// The load factor is the host's bound of it (after the inserts of this call); a bound
+// above the table's size says nothing, and counts as a low one.
+static unsigned bulk_spread(BulkOp op, bool p32, uint64_t bytes, double lf) {
+  const uint64_t mib = bytes >> 20;
+  if (mib < 16) return 0;
+  if (op == BulkOp::FIND) {
+    if (lf >= 0.9) return mib >= 128 ? 16 : 4;
+    if (lf >= 0.85) return mib >= 256 ? 6 : (mib >= 128 ? 4 : (p32 ? 0 : 2));
+    if (lf >= 0.75) return mib >= 256 ? 3 : 0;
+    return mib >= (p32 ? 512 : 2048) ? 2 : 0;
+  }
+  if (op == BulkOp::ERASE) {
+    if (lf >= 0.85) return 16;
+    if (lf >= 0.7) return mib >= 256 ? 16 : (mib >= 128 ? 8 : 0);
+    return mib >= 256 ? 8 : (mib >= 128 ? 4 : 0);
+  }
+  if (lf >= 0.85) return mib >= 512 ? 16 : (mib >= 128 ? 6 : (lf >= 0.88 ? 4 : 0));
+  if (lf >= 0.7) return mib >= 512 ? 8 : (mib >= 128 ? 4 : 0);
+  return mib >= 128 ? 4 : 0;
+}
 static bool bulk_pays(const BulkCall& c) {
   const uint64_t slots = 1ull << c.sp, bytes = (uint64_t)(c.key_bytes * 2) << c.sp;
   const int bits = c.sp - (c.key_bytes == 4 ? slice_log<P32>() : slice_log<P64>());
   if (bits < 1 || bits > 2 * kMaxDigitLog) return false;
-  if (HX_BULK_ALWAYS) return true;
   const double lf = c.fill_bound <= slots ? (double)c.fill_bound / (double)slots : 0.0;
-  const bool find = c.op == BulkOp::FIND;
-  unsigned spread = 0;
-  if (bytes >= (128ull << 20)) {
-    if (lf >= 0.85) spread = 16;
-    else if (lf >= 0.7) spread = find ? 4 : 8;
-    else spread = !find ? 4 : (c.key_bytes == 4 ? 2 : 0);
-  } else if (bytes >= (16ull << 20)) {
-    if (lf >= 0.85) spread = 4;
-    else if (lf >= 0.7) spread = 2;
-  }
+  const unsigned spread = bulk_spread(c.op, c.key_bytes == 4, bytes, lf);
   return spread && c.expected >= slots / spread;
 }
 

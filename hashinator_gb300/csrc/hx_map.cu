@@ -191,6 +191,9 @@ __device__ __forceinline__ bool cas_empty(P* b, typename PairTraits<P>::K& ek, t
 
 // BLIND: CAS the home bucket first without reading it (EMPTY buckets hold
 // (EMPTY, 0)); else load every key's first window, then CAS into it.
+#ifndef HX_LANES_MINB
+#define HX_LANES_MINB 5  // blocks per SM: 40 registers; 6 and 8 measured the same or slower
+#endif
 template <class P, int B, int U, bool PAIRS, bool BLIND>
 __global__ void __launch_bounds__(256) k_insert_t1(const typename PairTraits<P>::K* __restrict__ keys,
                                                    const typename PairTraits<P>::V* __restrict__ vals,
@@ -311,6 +314,254 @@ __global__ void __launch_bounds__(256) k_insert_t1(const typename PairTraits<P>:
   publish_counts(info, ins, maxd, fail, lane);
 }
 
+// ---- automatic thread-per-key kernels: first access, then a queue --------------
+// Most keys are decided by their first access. The others would hold up their warp's
+// 32 lanes for as long as the longest of them probes, and the code of a probe's later
+// steps would run for the few lanes that need it; so they go to a queue of the warp in
+// shared memory, and whenever it holds 32 keys, one probe step is run for 32 of them
+// at once. What is still open goes back to the queue. Bound by instructions and L2
+// round trips in tables that fit L2, by random DRAM sectors above: 4.2 M u32 inserts into
+// 2^23 empty buckets 106 us with one key per lane to its end (k_insert_t1), 97 us with
+// lanes that take their next key when done (250 instructions a turn), 76 us so.
+constexpr unsigned kQueue = 64;  // entries per warp: fewer than 32 wait while 32 more arrive
+
+// Buckets of the 32-byte window that holds bucket b, from b on: those equal to key, and
+// the EMPTY ones, as bits.
+template <class P, int B>
+__device__ __forceinline__ void window_bits(const Window<P, B>& w, typename PairTraits<P>::K key, uint32_t b,
+                                            unsigned& match, unsigned& empty) {
+  match = empty = 0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    match |= (unsigned)(w.k[j] == key) << j;
+    empty |= (unsigned)(w.k[j] == PairTraits<P>::EMPTY) << j;
+  }
+  const unsigned from = ~0u << (b & (B - 1));
+  match &= from;
+  empty &= from;
+}
+
+template <class P, int B, bool PAIRS>
+__global__ void __launch_bounds__(256, HX_LANES_MINB) k_insert_queue(const typename PairTraits<P>::K* __restrict__ keys,
+                                                                    const typename PairTraits<P>::V* __restrict__ vals,
+                                                                    const P* __restrict__ pairs, uint64_t n, P* table,
+                                                                    int sp, DInfo* info) {
+  using K = typename PairTraits<P>::K;
+  using V = typename PairTraits<P>::V;
+  constexpr K EMPTY = PairTraits<P>::EMPTY;
+  __shared__ P s_pair[8][kQueue];
+  __shared__ uint32_t s_b[8][kQueue];  // the bucket that the probe goes on from
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t tmask = (1u << sp) - 1u;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  P next;  // the next key, fetched ahead
+  auto fetch = [&]() {
+    next.first = EMPTY;
+    if (i < n) {
+      if constexpr (PAIRS) {
+        next = pairs[i];
+      } else {
+        next.first = keys[i];
+        next.second = vals ? vals[i] : (V)i;  // no values: insertIndex
+      }
+    }
+  };
+  fetch();
+  unsigned ins = 0, maxd = 0, queued = 0;
+  bool fail = false;
+  // One step of the probe of pr, at bucket b; whether it goes on (then from the new b).
+  auto step = [&](const P& pr, uint32_t& b) -> bool {
+    Window<P, B> w;
+    const uint32_t w0 = b & ~(uint32_t)(B - 1);
+    load_buckets<B>(table + w0, w.k, w.v);
+    unsigned match, empty;
+    window_bits<P, B>(w, pr.first, b, match, empty);
+    if (match) {
+      store_value(table + w0 + __ffs(match) - 1, pr.second);
+      return false;
+    }
+    const uint32_t h = home_slot(pr.first, sp);
+    uint32_t to = w0 + B;  // where the probe goes on
+    if (empty) {
+      const unsigned j = __ffs(empty) - 1;
+      K ek = EMPTY;
+      V ev{};
+#pragma unroll
+      for (int t = 0; t < B; ++t)
+        if (t == (int)j) ev = w.v[t];
+      to = w0 + j;
+      if (cas_pair(table + to, ek, ev, pr.first, pr.second)) {
+        ++ins;
+        maxd = max(maxd, ((to - h) & tmask) + 1);
+        return false;
+      }
+      if (ek == pr.first) {
+        store_value(table + to, pr.second);
+        return false;
+      }
+      if (ek != EMPTY) ++to;  // another key took it (else: EMPTY with another value, tried again)
+    }
+    if (((b - h) & tmask) + (to - b) > tmask) {  // round the whole table: no bucket is left
+      fail = true;
+      return false;
+    }
+    b = to & tmask;
+    return true;
+  };
+  for (;;) {
+    const bool more = __any_sync(0xffffffffu, i < n);
+    P pr;
+    uint32_t b = 0;
+    bool open = false;
+    if (more && queued < 32) {
+      pr = next;
+      i += stride;
+      fetch();
+      bool act = pr.first != EMPTY && pr.first != PairTraits<P>::TOMB;
+      // A key repeated within the warp is inserted once, by its lowest lane: the
+      // copies would only contend for the same bucket, and which of their values
+      // wins is unspecified anyway (a batch with duplicate keys races in the
+      // reference too). 2^20 keys plus 2^20 copies of one key insert an order of
+      // magnitude faster for it.
+      const unsigned held = __ballot_sync(0xffffffffu, act);
+      if (act) act = (__ffs(__match_any_sync(held, pr.first)) - 1) == lane;
+      if (act) {
+        b = home_slot(pr.first, sp);
+        K ek = EMPTY;
+        V ev = 0;  // what EMPTY buckets hold
+        if (cas_pair(table + b, ek, ev, pr.first, pr.second)) {
+          ++ins;
+          maxd = max(maxd, 1u);
+        } else if (ek == pr.first) {
+          store_value(table + b, pr.second);
+        } else {
+          open = true;
+          if (ek != EMPTY) b = (b + 1) & tmask;  // else EMPTY with a stale value: the window tells it
+        }
+      }
+    } else {
+      if (queued == 0) break;
+      const unsigned take = queued < 32 ? queued : 32;
+      queued -= take;
+      if ((unsigned)lane < take) {
+        pr = s_pair[wi][queued + lane];
+        b = s_b[wi][queued + lane];
+        open = step(pr, b);
+        while (open && !more && queued == 0) open = step(pr, b);  // the last ones: nothing to wait for
+      }
+      __syncwarp();
+    }
+    const unsigned wait = __ballot_sync(0xffffffffu, open);
+    if (open) {
+      const unsigned at = queued + __popc(wait & below);
+      s_pair[wi][at] = pr;
+      s_b[wi][at] = b;
+    }
+    queued += __popc(wait);
+    __syncwarp();
+  }
+  publish_counts(info, ins, maxd, fail, lane);
+}
+
+// retrieve and erase the same way: the first access is the window from the home bucket on.
+template <class P, int B, bool PAIRS, bool ERASE>
+__global__ void __launch_bounds__(256, HX_LANES_MINB) k_find_queue(const typename PairTraits<P>::K* __restrict__ keys,
+                                                                  typename PairTraits<P>::V* __restrict__ vals, P* pairs,
+                                                                  uint64_t n, P* table, int sp, DInfo* info) {
+  using K = typename PairTraits<P>::K;
+  using V = typename PairTraits<P>::V;
+  const unsigned limit = info->max_probe;
+  if (limit == 0) return;
+  __shared__ K s_key[8][kQueue];
+  __shared__ uint32_t s_b[8][kQueue];
+  __shared__ uint64_t s_i[8][kQueue];  // where its value goes
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t tmask = (1u << sp) - 1u;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  auto fetch = [&]() -> K {
+    if (i >= n) return PairTraits<P>::EMPTY;
+    if constexpr (PAIRS) return pairs[i].first;
+    else return keys[i];
+  };
+  K next = fetch();
+  unsigned erased = 0, queued = 0;
+  auto step = [&](K key, uint64_t at, uint32_t& b) -> bool {
+    Window<P, B> w;
+    const uint32_t w0 = b & ~(uint32_t)(B - 1);
+    load_buckets<B>(table + w0, w.k, w.v);
+    unsigned match, empty;
+    window_bits<P, B>(w, key, b, match, empty);
+    if (match) {
+      const unsigned j = __ffs(match) - 1;
+      if constexpr (ERASE) {
+        if (cas_key(table + w0 + j, key, PairTraits<P>::TOMB)) ++erased;
+      } else {
+        V v{};
+#pragma unroll
+        for (int t = 0; t < B; ++t)
+          if (t == (int)j) v = w.v[t];
+        if constexpr (PAIRS) pairs[at].second = v;
+        else vals[at] = v;
+      }
+      return false;
+    }
+    if (empty) return false;
+    // past the longest probe of any key (which is at most the table)
+    const uint32_t d = ((b - home_slot(key, sp)) & tmask) + (w0 + B - b);
+    b = (w0 + B) & tmask;
+    return d < limit;
+  };
+  for (;;) {
+    const bool more = __any_sync(0xffffffffu, i < n);
+    K key{};
+    uint64_t at = 0;
+    uint32_t b = 0;
+    bool open = false;
+    if (more && queued < 32) {
+      key = next;
+      at = i;
+      i += stride;
+      next = fetch();
+      if (key != PairTraits<P>::EMPTY && key != PairTraits<P>::TOMB) {
+        b = home_slot(key, sp);
+        open = step(key, at, b);
+      }
+    } else {
+      if (queued == 0) break;
+      const unsigned take = queued < 32 ? queued : 32;
+      queued -= take;
+      if ((unsigned)lane < take) {
+        key = s_key[wi][queued + lane];
+        b = s_b[wi][queued + lane];
+        at = s_i[wi][queued + lane];
+        open = step(key, at, b);
+        while (open && !more && queued == 0) open = step(key, at, b);
+      }
+      __syncwarp();
+    }
+    const unsigned wait = __ballot_sync(0xffffffffu, open);
+    if (open) {
+      const unsigned q = queued + __popc(wait & below);
+      s_key[wi][q] = key;
+      s_b[wi][q] = b;
+      s_i[wi][q] = at;
+    }
+    queued += __popc(wait);
+    __syncwarp();
+  }
+  if constexpr (ERASE) {
+    erased = __reduce_add_sync(0xffffffffu, erased);
+    if (lane == 0 && erased) {
+      atomicAdd(&info->tombstones, (unsigned long long)erased);
+      atomicAdd(&info->fill, 0ull - (unsigned long long)erased);
+    }
+  }
+}
+
 template <class P, int B, int U, bool PAIRS, bool ERASE>
 __global__ void __launch_bounds__(256) k_find_t1(const typename PairTraits<P>::K* __restrict__ keys,
                                                  typename PairTraits<P>::V* __restrict__ vals, P* pairs, uint64_t n,
@@ -414,17 +665,26 @@ static inline unsigned key_bytes(const hx_map* m) { return is_p32(m) ? 4u : 8u; 
 static inline uint64_t nslots(const hx_map* m) { return 1ull << m->sp; }
 
 // Automatic probe policy (tune.group == 0), from GB300 sweeps over
-// G x keys-per-thread at load factors 0.5 - 0.9 (2^27 buckets, u32 and u64):
-//   insert:  one thread per key, blind home CAS, 1 key per thread, unless
-//            the insert ends above load factor 0.85: then 4-lane groups
-//            (u32 11.9 vs 10.9, u64 7.1 vs 6.9 G keys/s at 0.9);
-//   query:   probe groups with the single-exit probe loop: u32 tables use
-//            4 lanes (64 B windows) below load factor 0.875 and 8 above (31.6
-//            vs 29.8 G keys/s for thread-per-key at 0.5, 7.9 vs 6.7 for 32
-//            lanes at 0.9); u64 tables 4 lanes below 0.8, 8 to 0.875, 16 above
-//            (24.8 vs 21.1 G keys/s for thread-per-key at 0.5, 12.9 vs 10.6 for
-//            16 lanes at 0.75);
-//   erase:   one thread per key with 2 keys in flight at every load factor
+// G x keys-per-thread at load factors 0.3 - 0.9 (2^14 - 2^27 buckets, u32 and u64):
+//   insert:  one thread per key, blind home CAS (1.9 M u32 keys into 2^23 buckets
+//            that end at 0.92: 241 against 423 us for 4-lane groups, u64 411 against
+//            862 us), except above 0.88 in tables over 512 MiB (2^27 u32 buckets
+//            from 0.86 to 0.92: 2.62 against 2.30 ms) and for fewer than 2^16 keys
+//            (15 K at 0.92: 50 against 44 us): 4-lane groups;
+//   query:   one thread per key (its 32-byte windows are the least traffic) below
+//            load factor 0.75: 2^20 u32 queries in 2^21 buckets at 0.5 16 us against
+//            39 us for 4-lane groups, u64 18 against 47 us; 2^26 buckets at 0.7,
+//            5.9 M u32 queries, 217 against 278 us. Above that:
+//            tables up to 128 MiB, which stay in L2: still one thread per key
+//            (2^23 u32 buckets at 0.8 77 against 145 us for 8 lanes), but 16 lanes
+//            where few keys with long probes do not fill the GPU (236 K u32
+//            queries at 0.9 44 against 65 us, 15 K 9 against 28 us) and for u64
+//            from 0.88 on (321 against 344 us);
+//            larger ones: u32 one thread per key to 0.875 (2^26 buckets at 0.8 371
+//            against 455 us), 8 lanes above (7.9 against 6.7 G keys/s for 32 lanes at
+//            0.9); u64 4 lanes below 0.8, 8 to 0.875 (2^27 buckets at 0.8 1.33
+//            against 1.51 ms for one thread per key), 16 above;
+//   erase:   one thread per key at every load factor
 //            (erased keys are usually present, so a probe ends at the key,
 //            not at the end of a long run; 1.1-2.7x faster than groups).
 enum class Op { INSERT, QUERY, ERASE };
@@ -434,21 +694,27 @@ struct Geo {
 struct Policy {
   int G, U;
 };
-static Policy auto_policy(const hx_map* m, Op op) {
+static Policy auto_policy(const hx_map* m, Op op, uint64_t n) {
   if (op == Op::INSERT) {
     // fill_ub already counts this call's keys: the load factor the insert ends at
     const double lf_end = (double)m->fill_ub / (double)nslots(m);
-    return lf_end < 0.85 ? Policy{1, 1} : Policy{4, 1};
+    const bool groups = lf_end >= 0.88 && (nslots(m) * pair_bytes(m) > (512ull << 20) || n < (1u << 16));
+    return groups ? Policy{4, 1} : Policy{1, 1};
   }
-  if (op == Op::ERASE) return {1, 2};
+  if (op == Op::ERASE) return {1, 1};
   const double lf = (double)m->fill_ub / (double)nslots(m);
   const bool p32 = is_p32(m);
-  if (p32) return lf < 0.875 ? Policy{4, 1} : Policy{8, 1};
+  if (lf < 0.75) return {1, 1};
+  if (nslots(m) * pair_bytes(m) <= (128ull << 20)) {
+    if (lf < 0.8) return {1, 1};
+    return n < (1u << 19) || (!p32 && lf >= 0.88) ? Policy{16, 1} : Policy{1, 1};
+  }
+  if (p32) return lf < 0.875 ? Policy{1, 1} : Policy{8, 1};
   if (lf < 0.8) return {4, 1};
   return lf < 0.875 ? Policy{8, 1} : Policy{16, 1};
 }
-static Policy policy(const hx_map* m, Op op) {
-  if (m->tune.group == 0) return auto_policy(m, op);
+static Policy policy(const hx_map* m, Op op, uint64_t n) {
+  if (m->tune.group == 0) return auto_policy(m, op, n);
   return {m->tune.group, m->tune.unroll};
 }
 
@@ -531,10 +797,21 @@ static hx_status launch_insert(hx_map* m, const void* keys, const void* vals, co
   // the device) into a table whose fill bound still counts the erased keys:
   // thread-per-key, and reading the window before any CAS, as such a key's home
   // is mostly taken.
-  const Policy pol = (d_n && m->tune.group == 0) ? Policy{1, 1} : policy(m, Op::INSERT);
+  const Policy pol = (d_n && m->tune.group == 0) ? Policy{1, 1} : policy(m, Op::INSERT, n);
   const bool blind = d_n ? false : m->tune.blind;
   const Geo geo = pick_geo(m, pol.G);
   const int block = m->tune.block;
+  constexpr int BT = sizeof(P) == 8 ? 4 : 2;
+  if (!d_n && m->tune.group == 0 && pol.G == 1 && blind && !m->tune.wide && nslots(m) >= 2 * BT) {
+    auto go = [&](auto kern) {
+      kern<<<grid_for(kern, n, block), block, 0, s>>>(static_cast<const K*>(keys), static_cast<const V*>(vals),
+                                                      static_cast<const P*>(pairs), n, static_cast<P*>(m->buckets),
+                                                      m->sp, m->info);
+    };
+    if (pairs) go(k_insert_queue<P, BT, true>);
+    else go(k_insert_queue<P, BT, false>);
+    return after_launch();
+  }
   if (geo.G == 1) {
     const int U = pol.U;
 #define HX_LAUNCH_INSERT_T1_B(PP, BB, UU, BL)                                                                     \
@@ -585,9 +862,20 @@ template <class P, bool ERASE>
 static hx_status launch_find(hx_map* m, const void* keys, void* vals, void* pairs, uint64_t n, cudaStream_t s) {
   using K = typename PairTraits<P>::K;
   using V = typename PairTraits<P>::V;
-  const Policy pol = policy(m, ERASE ? Op::ERASE : Op::QUERY);
+  const Policy pol = policy(m, ERASE ? Op::ERASE : Op::QUERY, n);
   const Geo geo = pick_geo(m, pol.G);
   const int block = m->tune.block;
+  constexpr int BT = sizeof(P) == 8 ? 4 : 2;
+  if (m->tune.group == 0 && pol.G == 1 && !m->tune.wide && nslots(m) >= 2 * BT) {
+    auto go = [&](auto kern) {
+      kern<<<grid_for(kern, n, block), block, 0, s>>>(static_cast<const K*>(keys), static_cast<V*>(vals),
+                                                      static_cast<P*>(pairs), n, static_cast<P*>(m->buckets), m->sp,
+                                                      m->info);
+    };
+    if (pairs) go(k_find_queue<P, BT, true, ERASE>);
+    else go(k_find_queue<P, BT, false, ERASE>);
+    return after_launch();
+  }
   if (geo.G == 1) {
     const int U = pol.U;
 #define HX_LAUNCH_FIND_T1(PP, BB, UU)                                                                            \

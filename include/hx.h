@@ -230,11 +230,11 @@ hx_status hx_map_device_view(hx_map* map, hx_device_view* out);
  * {1,2,4,8,16,32} lanes per key (1 = one thread per key with
  * keys_per_thread in {1,2,4,8} keys in flight), applied to insert, retrieve
  * and erase alike; block_size a multiple of 32 up to 256. 0 keeps the
- * current value. Until a group width is set, each call picks its own: one
- * thread per key for erase, for the re-insert of clean_tombstones and for
- * an insert whose load factor ends below 0.85 (4-lane groups above); small
- * probe groups for retrieve (u32: 4 lanes below load factor 0.875, 8 above;
- * u64: 4 below 0.8, 8 to 0.875, 16 above). */
+ * current value. Until a group width is set, each call picks its own: large
+ * batches on large or dense tables go slice by slice through the table; others
+ * use one thread per key, except inserts that end above load factor 0.88 and
+ * look-ups above 0.75 - 0.875 where probe groups of 4 - 16 lanes are faster
+ * (by table size, key width and batch size). */
 hx_status hx_map_set_tuning(hx_map* map, int group_width, int keys_per_thread, int block_size);
 
 /* Thread-per-key insert mode (no reference counterpart): blind_cas != 0
