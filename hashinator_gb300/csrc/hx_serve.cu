@@ -293,6 +293,8 @@ struct ServeMap {
   uint64_t in_flight = 0;        // inserts launched in rounds not yet completed
   uint64_t in_flight_erase = 0;  // erase keys launched in rounds not yet completed
   uint64_t rehash_round = 0;     // first round that runs on the current table
+  unsigned base_probe = 0;       // longest probe of the first snapshot of the current table (0: none yet)
+  bool tangled = false;          // its probes run long through tombstones
 };
 
 struct Pending {
@@ -364,6 +366,18 @@ static void view_of(hx_server* sv, unsigned i, hx_map* v) {
   v->fill_ub = sv->maps[i].fill_ub;
 }
 
+// Keys that come and go leave their tombstones behind one another from their homes on,
+// and a probe to such a home passes all of them, long before the table is full: rounds
+// that insert and erase the same keys took 1.1 ms at first and 7 ms after 200 rounds
+// (256 maps, 3.1 M keys; with this rule 1.1 ms, with a bound of 128 or 256 buckets 1.1 /
+// 1.2 ms). A map whose longest probe passed
+// kLongProbe buckets and twice what it was on the fresh table, with tombstones enough to
+// account for it, is rehashed at its size before its next round, which drops them.
+#ifndef HX_SERVE_LONG_PROBE
+#define HX_SERVE_LONG_PROBE 64
+#endif
+constexpr unsigned kLongProbe = HX_SERVE_LONG_PROBE;
+
 // Completed rounds: completion times, fill bounds refreshed from the
 // round's metadata snapshot.
 static hx_status reap(hx_server* sv, bool wait_oldest) {
@@ -393,7 +407,12 @@ static hx_status reap(hx_server* sv, bool wait_oldest) {
       ServeMap& m = sv->maps[i];
       m.fill_ub = sl.h_info[i].fill + m.in_flight;  // a rehash keeps fill
       // tombstones of a snapshot taken before the map's last rehash are gone
-      if (sl.round_no >= m.rehash_round) m.tomb_ub = sl.h_info[i].tombstones + m.in_flight_erase;
+      if (sl.round_no >= m.rehash_round) {
+        m.tomb_ub = sl.h_info[i].tombstones + m.in_flight_erase;
+        const unsigned probe = sl.h_info[i].max_probe;
+        if (m.base_probe == 0) m.base_probe = probe;
+        m.tangled = probe > kLongProbe && probe > 2 * m.base_probe && sl.h_info[i].tombstones * 4 > probe;
+      }
     }
     sl.busy = false;
     sl.tags.clear();
@@ -595,14 +614,44 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
   std::vector<GrowTask> tasks;
   std::vector<void*> old_tables;
   const uint64_t this_round = sv->rounds;
+  // One batched rehash per map and round: a second need in the same round replaces
+  // the pending target with the larger table.
+  auto schedule = [&](uint32_t map, int nsp) -> hx_status {
+    ServeMap& m = sv->maps[map];
+    const uint64_t nbytes = (1ull << nsp) * pb(sv);
+    int& slot_of = grow_of[map];
+    void* nt = nullptr;
+    HX_CUDA(cudaMallocFromPoolAsync(&nt, nbytes, sv->pool, sv->s));
+    if (slot_of < 0) {
+      slot_of = (int)tasks.size();
+      tasks.push_back(GrowTask{m.table, nt, 1ull << m.sp, nsp, map});
+      old_tables.push_back(m.table);
+    } else {
+      HX_CUDA(cudaFreeAsync(tasks[slot_of].new_table, sv->s));  // never used
+      tasks[slot_of].new_table = nt;
+      tasks[slot_of].new_sp = nsp;
+    }
+    sv->used = sv->used - m.bytes + nbytes;
+    sv->st.growths++;
+    sv->st.growth_bytes += nbytes;
+    m.table = nt;
+    m.sp = nsp;
+    m.bytes = nbytes;
+    m.tomb_ub = 0;
+    m.tangled = false;
+    m.base_probe = 0;
+    m.rehash_round = this_round;
+    return HX_OK;
+  };
   for (size_t i = 0; i < round.size(); ++i) {
     const hx_request& r = round[i].r;
+    ServeMap& m = sv->maps[r.map];
+    if (m.tangled && r.n && (st = schedule(r.map, m.sp)) != HX_OK) return st;
     if (r.op == SOP_ERASE) {
       era[r.map] += r.n;
       continue;
     }
     if (r.op != SOP_INSERT || r.n == 0) continue;
-    ServeMap& m = sv->maps[r.map];
     const double lim = (double)sv->max_lf;
     const uint64_t occ = m.fill_ub + m.tomb_ub + add[r.map] + era[r.map] + r.n;
     if ((double)occ > lim * (double)(1ull << m.sp)) {
@@ -615,28 +664,7 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
         admitted[i] = 0;  // cannot make room within the budget: reject this insert
         continue;
       }
-      // one batched rehash per map and round: a second need in the same round
-      // replaces the pending target with the larger table
-      int& slot_of = grow_of[r.map];
-      void* nt = nullptr;
-      HX_CUDA(cudaMallocFromPoolAsync(&nt, nbytes, sv->pool, sv->s));
-      if (slot_of < 0) {
-        slot_of = (int)tasks.size();
-        tasks.push_back(GrowTask{m.table, nt, 1ull << m.sp, nsp, r.map});
-        old_tables.push_back(m.table);
-      } else {
-        HX_CUDA(cudaFreeAsync(tasks[slot_of].new_table, sv->s));  // never used
-        tasks[slot_of].new_table = nt;
-        tasks[slot_of].new_sp = nsp;
-      }
-      sv->used = sv->used - m.bytes + nbytes;
-      sv->st.growths++;
-      sv->st.growth_bytes += nbytes;
-      m.table = nt;
-      m.sp = nsp;
-      m.bytes = nbytes;
-      m.tomb_ub = 0;
-      m.rehash_round = this_round;
+      if ((st = schedule(r.map, nsp)) != HX_OK) return st;
     }
     add[r.map] += r.n;
   }
