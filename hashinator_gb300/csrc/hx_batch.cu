@@ -82,31 +82,43 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Waits until *p == 0, for about one second at most.
-__device__ __forceinline__ bool wait_zero(const unsigned* p) {
-  if (ld_acquire_u32(p) == 0) return true;
+// Waits until the counters p[0], p[stride], .. p[(n - 1) * stride] are all 0, for about
+// one second at most: one counter per lane of the calling warp, read side by side.
+__device__ __forceinline__ bool wait_zero(const unsigned* p, unsigned stride, unsigned n, int lane) {
+  auto zero = [&]() { return __all_sync(0xffffffffu, (unsigned)lane >= n || ld_acquire_u32(p + lane * stride) == 0); };
+  if (zero()) return true;
   const unsigned long long t0 = global_ns();
   for (unsigned i = 0; i < kBatchSpinLimit; ++i) {
     __nanosleep(i < 32 ? 32 : 256);
-    if (ld_acquire_u32(p) == 0) return true;
-    if ((i & 63) == 63 && global_ns() - t0 > kBatchWaitNs) return false;
+    if (zero()) return true;
+    const bool late = (i & 63) == 63 && global_ns() - t0 > kBatchWaitNs;
+    if (__any_sync(0xffffffffu, late)) return false;
   }
   return false;
 }
 
+// A key whose probe waits for its next step, at bucket b (queue_run).
+template <class P>
+struct InsertRec {
+  P pr;
+  uint32_t b;
+};
+template <class P>
+struct FindRec {
+  typename PairTraits<P>::K key;
+  uint32_t b, k;  // k: its number in the tile
+};
+
 template <class P, int G, int BLOCK>
 // The round is bound by memory-level parallelism (random probes of many small
-// tables), not by DRAM bytes: capping registers so that 48 warps fit per SM
-// (some spills to L1) took it from about 4.5 to 3.2 ms against 20 warps at 96
-// registers (sweep of 20/24/32/40/48/64 warps on GB300).
+// tables) and by instructions, not by DRAM bytes. With one key per lane to its end,
+// 48 warps per SM were best (4096 maps, 39 M keys: 3.21 ms a round); with the probes
+// that go on in queues (queue_run) 64 warps are, at 32 registers (some spill to L1):
+// 2.03 ms, 48 warps 2.30, 40 2.57, 32 2.91. Waiting for a tile's earlier phases with one
+// lane per phase instead of one after the other, and four times the keys per
+// re-insert tile, took it to 1.94 ms.
 #ifndef HX_BATCH_MIN_WARPS
-#define HX_BATCH_MIN_WARPS 48
-#endif
-// Inserts per thread whose first CAS is in flight at once. One key at a time
-// measured fastest on GB300 (2.99 ms a round): 2 in flight at 48 warps per SM
-// took 3.13 ms, 2 or 4 at 32 warps 3.34 / 3.41 ms.
-#ifndef HX_BATCH_INSERTS_IN_FLIGHT
-#define HX_BATCH_INSERTS_IN_FLIGHT 1
+#define HX_BATCH_MIN_WARPS 64
 #endif
 __global__ void __launch_bounds__(BLOCK, HX_BATCH_MIN_WARPS * 32 / BLOCK > 0 ? HX_BATCH_MIN_WARPS * 32 / BLOCK : 1)
     k_batch(BatchArgs<P> a) {
@@ -116,25 +128,29 @@ __global__ void __launch_bounds__(BLOCK, HX_BATCH_MIN_WARPS * 32 / BLOCK > 0 ? H
   constexpr K TOMB = PairTraits<P>::TOMB;
   constexpr int BT = sizeof(P) == 8 ? 4 : 2;  // thread-per-key window: 32 B
   constexpr int BG = sizeof(P) == 8 ? 2 : 1;  // group lane: 16 B
-  constexpr int U = 4;                        // lookups in flight per thread
-  constexpr int UI = HX_BATCH_INSERTS_IN_FLIGHT;  // inserts in flight per thread
   __shared__ Tile s_t;
   __shared__ unsigned s_ok, s_ins, s_max, s_fail, s_erased, s_moved;
+  __shared__ union {  // the warps' queues, of one phase at a time
+    InsertRec<P> ins[BLOCK / 32][kQueue];
+    FindRec<P> find[BLOCK / 32][kQueue];
+  } s_queue;
   const int lane = threadIdx.x & 31;
   for (;;) {
-    if (threadIdx.x == 0) {
-      const unsigned idx = atomicAdd(a.work, 1u);
+    if (threadIdx.x < 32) {
       Tile t;
-      if (idx < a.n_tiles) t = a.tiles[idx];
-      else t.map = 0xffffffffu;
-      s_t = t;
-      s_ins = s_max = s_fail = s_erased = s_moved = 0;
-      unsigned ok = 1;
-      if (t.map != 0xffffffffu) {
-        for (int q = (int)t.phase - 1; q >= 0 && ok; --q) ok = wait_zero(a.remaining + q * a.n_maps + t.map);
-        if (!ok) atomicExch(a.error, 1u);
+      if (lane == 0) {
+        const unsigned idx = atomicAdd(a.work, 1u);
+        if (idx < a.n_tiles) t = a.tiles[idx];
+        else t.map = 0xffffffffu;
+        s_t = t;
+        s_ins = s_max = s_fail = s_erased = s_moved = 0;
+        s_ok = 1;
       }
-      s_ok = ok;
+      const unsigned map = __shfl_sync(0xffffffffu, t.map, 0), phase = __shfl_sync(0xffffffffu, t.phase, 0);
+      if (map != 0xffffffffu && !wait_zero(a.remaining + map, a.n_maps, phase, lane) && lane == 0) {
+        s_ok = 0;
+        atomicExch(a.error, 1u);
+      }
     }
     __syncthreads();
     const Tile t = s_t;
@@ -163,28 +179,34 @@ __global__ void __launch_bounds__(BLOCK, HX_BATCH_MIN_WARPS * 32 / BLOCK > 0 ? H
           }
           // inserts are thread-per-key whatever the tuned group width: on
           // GB300 they measured fastest at every load factor
-          auto load = [&](unsigned k, K& key, V& val) {
-            if (src) {
-              const P pr = src[begin + k];
-              key = pr.first;
-              val = pr.second;
-            } else {
-              key = a.ins_keys[begin + k];
-              val = a.ins_vals[begin + k];
-            }
-          };
           const unsigned cnt = (unsigned)count;
-          if (src) {  // moved keys, whose homes are mostly taken: window first, as the single-map clean
-            for (unsigned k = threadIdx.x; k < cnt; k += BLOCK) {
-              K key;
-              V val;
-              load(k, key, val);
-              insert_one_t1_win<P, BT>(tab, sp, key, val, ins, maxd, fail);
-            }
-          } else {
-            for (unsigned base = 0; base < cnt; base += BLOCK * UI)
-              insert_t1_many<P, BT, UI>(tab, sp, base + threadIdx.x, BLOCK, cnt, load, ins, maxd, fail);
-          }
+          auto step = [&](InsertRec<P>& q) { return insert_step<P, BT>(tab, sp, q.pr, q.b, ins, maxd, fail); };
+          queue_run(s_queue.ins[threadIdx.x / 32], threadIdx.x & ~31u, BLOCK, cnt, lane,
+                    [&](unsigned k, InsertRec<P>& q) -> bool {
+                      if (src) {  // moved keys, whose homes are mostly taken: the window before any CAS
+                        q.pr = src[begin + k];
+                        q.b = home_slot(q.pr.first, sp);
+                        return step(q);
+                      }
+                      q.pr.first = a.ins_keys[begin + k];
+                      q.pr.second = a.ins_vals[begin + k];
+                      if (q.pr.first == EMPTY || q.pr.first == TOMB) return false;
+                      q.b = home_slot(q.pr.first, sp);
+                      K ek = EMPTY;
+                      V ev = 0;  // what EMPTY buckets hold
+                      if (cas_pair(tab + q.b, ek, ev, q.pr.first, q.pr.second)) {
+                        ++ins;
+                        maxd = max(maxd, 1u);
+                        return false;
+                      }
+                      if (ek == q.pr.first) {
+                        store_value(tab + q.b, q.pr.second);
+                        return false;
+                      }
+                      if (ek != EMPTY) q.b = (q.b + 1) & ((1u << sp) - 1u);  // else: a stale value, the window tells it
+                      return true;
+                    },
+                    step);
           break;
         }
         case BP_QUERY:
@@ -195,38 +217,28 @@ __global__ void __launch_bounds__(BLOCK, HX_BATCH_MIN_WARPS * 32 / BLOCK > 0 ? H
           if (limit == 0) break;
           // the tuned group width applies to queries; erases are thread-per-key
           if (!groups || erase) {
-            for (unsigned base = 0; base < t.count; base += BLOCK * U) {
-              K key[U];
-              bool act[U];
-              uint32_t h[U];
-              Window<P, BT> w[U];
-#pragma unroll
-              for (int u = 0; u < U; ++u) {
-                const unsigned k = base + u * BLOCK + threadIdx.x;
-                act[u] = k < t.count;
-                if (act[u]) {
-                  key[u] = keys[t.begin + k];
-                  act[u] = key[u] != EMPTY && key[u] != TOMB;
-                }
-                if (act[u]) {
-                  h[u] = home_slot(key[u], sp);
-                  load_buckets<BT>(tab + (h[u] & ~(uint32_t)(BT - 1)), w[u].k, w[u].v);
+            auto step = [&](FindRec<P>& q) -> bool {
+              uint32_t slot;
+              V v;
+              const int r = find_step<P, BT>(tab, sp, limit, q.key, q.b, slot, v);
+              if (r == FS_HIT) {
+                if (erase) {
+                  if (cas_key(tab + slot, q.key, TOMB)) ++erased;
+                } else {
+                  a.q_out[t.begin + q.k] = v;
                 }
               }
-#pragma unroll
-              for (int u = 0; u < U; ++u) {
-                if (!act[u]) continue;
-                uint32_t slot;
-                V v;
-                if (find_t1<P, BT>(tab, sp, key[u], limit, h[u], w[u], slot, v)) {
-                  if (erase) {
-                    if (cas_key(tab + slot, key[u], TOMB)) ++erased;
-                  } else {
-                    a.q_out[t.begin + base + u * BLOCK + threadIdx.x] = v;
-                  }
-                }
-              }
-            }
+              return r == FS_ON;
+            };
+            queue_run(s_queue.find[threadIdx.x / 32], threadIdx.x & ~31u, BLOCK, t.count, lane,
+                      [&](unsigned k, FindRec<P>& q) -> bool {
+                        q.key = keys[t.begin + k];
+                        if (q.key == EMPTY || q.key == TOMB) return false;
+                        q.k = k;
+                        q.b = home_slot(q.key, sp);
+                        return step(q);
+                      },
+                      step);
           } else if constexpr (G > 1) {
             const unsigned gmask = group_mask<G>(lane);
             for (unsigned k = threadIdx.x / G; k < t.count; k += BLOCK / G) {
@@ -325,18 +337,10 @@ __global__ void __launch_bounds__(BLOCK, HX_BATCH_MIN_WARPS * 32 / BLOCK > 0 ? H
   }
 }
 
+// Every bucket (EMPTY, 0) and every map's metadata as an empty map's.
 template <class P>
-__global__ void k_batch_fill_empty(P* arena, uint64_t n) {
-  P e;
-  e.first = PairTraits<P>::EMPTY;
-  e.second = 0;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    arena[i] = e;
-}
-
-__global__ void k_batch_info_reset(DInfo* info, unsigned n) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
+__global__ void k_batch_clear(P* arena, uint64_t n, DInfo* info, unsigned maps) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < maps; i += gridDim.x * blockDim.x) {
     info[i].fill = 0;
     info[i].tombstones = 0;
     info[i].max_probe = 0;
@@ -346,6 +350,11 @@ __global__ void k_batch_info_reset(DInfo* info, unsigned n) {
     info[i].done = info[i].max_next = 0;
     info[i].left_next = info[i].moved_next = info[i].left = 0;
   }
+  P e;
+  e.first = PairTraits<P>::EMPTY;
+  e.second = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    arena[i] = e;
 }
 
 }  // namespace hx
@@ -370,6 +379,7 @@ struct hx_batch_plan {
   hx_batch_work w{};
   std::vector<uint64_t> ins_off, q_off, e_off;
   int group = 1, block = 256, tile = 2048;
+  bool tile_set = false;  // by the caller or the autotuner
   unsigned n_tiles = 0;
   hx::Tile* d_tiles = nullptr;
   unsigned* d_counters = nullptr;  // [0]: ticket, [1]: error, [2..]: remaining
@@ -400,6 +410,18 @@ static void free_plan_device(hx_batch_plan* p) {
   p->d_remaining_init = nullptr;
 }
 
+// Keys per tile: the tuned size; until one is set, 2048, or as many fewer (512 at least)
+// as give two tiles per SM in the largest phase (300 K keys on 100 maps: a round takes
+// 151 us with 2048 keys, 113 us with 512).
+static int tile_keys(const hx_batch_plan* p) {
+  if (p->tile_set) return p->tile;
+  auto keys = [](const std::vector<uint64_t>& o) { return o.empty() ? 0 : o.back() - o.front(); };
+  const uint64_t most = std::max(keys(p->ins_off), std::max(keys(p->q_off), keys(p->e_off)));
+  int t = p->tile;
+  while (t > 512 && most / t < 2 * (uint64_t)sm_count()) t /= 2;
+  return t;
+}
+
 // Builds the tile list and the per-map phase counters on the host, uploads
 // them. Phase-major order; inside a phase, larger maps first.
 static hx_status build_tiles(hx_batch_plan* p, cudaStream_t s) {
@@ -411,7 +433,7 @@ static hx_status build_tiles(hx_batch_plan* p, cudaStream_t s) {
   std::vector<unsigned> order(nm);
   for (unsigned i = 0; i < nm; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(), [&](unsigned x, unsigned y) { return b->sp[x] > b->sp[y]; });
-  const uint64_t T = (uint64_t)p->tile;
+  const uint64_t T = (uint64_t)tile_keys(p);
   // Maps in groups of consecutive maps (largest first) whose tables total
   // about kGroupBytes (24 MiB), and each group's phases software-pipelined across the
   // tile list: group g's inserts, then g-1's queries, g-2's erases, g-3's
@@ -446,6 +468,11 @@ static hx_status build_tiles(hx_batch_plan* p, cudaStream_t s) {
       }
     }
   };
+  // Re-insert tiles are laid out for the bound of moved keys, of which a fifth is usual:
+  // four times the keys per tile, unless that would leave SMs without one.
+  uint64_t most_moved = 0;
+  for (unsigned i = 0; i < nm; ++i) most_moved += p->moved_cap[i];
+  const uint64_t TR = most_moved / T >= 64 * (uint64_t)sm_count() ? 4 * T : T;
   const long ng = (long)groups.size();
   for (long step = 0; step < ng + 4; ++step) {
     if (step < ng) add_segments(BP_INSERT, p->ins_off, groups[step]);
@@ -469,8 +496,8 @@ static hx_status build_tiles(hx_batch_plan* p, cudaStream_t s) {
     }
     if (step - 4 >= 0 && step - 4 < ng) {
       for (unsigned i : groups[step - 4]) {
-        for (uint64_t a0 = 0; a0 < p->moved_cap[i]; a0 += T) {
-          tiles.push_back(Tile{i, BP_CLEAN_REINSERT, a0, (unsigned)T, 0});
+        for (uint64_t a0 = 0; a0 < p->moved_cap[i]; a0 += TR) {
+          tiles.push_back(Tile{i, BP_CLEAN_REINSERT, a0, (unsigned)TR, 0});
           rem[(size_t)BP_CLEAN_REINSERT * nm + i]++;
         }
       }
@@ -631,11 +658,10 @@ hx_status hx_batch_clear(hx_batch* b, hx_stream stream) {
   if (!b) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned grid = (unsigned)(sm_count() * 8);
-  if (b->key_bytes == 4) k_batch_fill_empty<P32><<<grid, 256, 0, s>>>(static_cast<P32*>(b->arena), b->total_buckets);
-  else k_batch_fill_empty<P64><<<grid, 256, 0, s>>>(static_cast<P64*>(b->arena), b->total_buckets);
-  hx_status st = after_launch();
-  if (st != HX_OK) return st;
-  k_batch_info_reset<<<(b->n_maps + 255) / 256, 256, 0, s>>>(b->d_info, b->n_maps);
+  if (b->key_bytes == 4)
+    k_batch_clear<P32><<<grid, 256, 0, s>>>(static_cast<P32*>(b->arena), b->total_buckets, b->d_info, b->n_maps);
+  else
+    k_batch_clear<P64><<<grid, 256, 0, s>>>(static_cast<P64*>(b->arena), b->total_buckets, b->d_info, b->n_maps);
   std::fill(b->fill_ub.begin(), b->fill_ub.end(), 0);
   return after_launch();
 }
@@ -738,8 +764,9 @@ hx_status hx_batch_set_tuning(hx_batch_plan* p, int group_width, int block_size,
   if (tile_keys && (tile_keys < 64 || tile_keys > (1 << 20))) return HX_ERR_INVALID_ARG;
   if (group_width) p->group = group_width;
   if (block_size) p->block = block_size;
-  if (tile_keys && tile_keys != p->tile) {
+  if (tile_keys && (tile_keys != p->tile || !p->tile_set)) {
     p->tile = tile_keys;
+    p->tile_set = true;
     return build_tiles(p, static_cast<cudaStream_t>(stream));
   }
   if (p->graph_exec) {  // the captured launch has the old tuning baked in

@@ -323,23 +323,6 @@ __global__ void __launch_bounds__(256) k_insert_t1(const typename PairTraits<P>:
 // round trips in tables that fit L2, by random DRAM sectors above: 4.2 M u32 inserts into
 // 2^23 empty buckets 106 us with one key per lane to its end (k_insert_t1), 97 us with
 // lanes that take their next key when done (250 instructions a turn), 76 us so.
-constexpr unsigned kQueue = 64;  // entries per warp: fewer than 32 wait while 32 more arrive
-
-// Buckets of the 32-byte window that holds bucket b, from b on: those equal to key, and
-// the EMPTY ones, as bits.
-template <class P, int B>
-__device__ __forceinline__ void window_bits(const Window<P, B>& w, typename PairTraits<P>::K key, uint32_t b,
-                                            unsigned& match, unsigned& empty) {
-  match = empty = 0;
-#pragma unroll
-  for (int j = 0; j < B; ++j) {
-    match |= (unsigned)(w.k[j] == key) << j;
-    empty |= (unsigned)(w.k[j] == PairTraits<P>::EMPTY) << j;
-  }
-  const unsigned from = ~0u << (b & (B - 1));
-  match &= from;
-  empty &= from;
-}
 
 template <class P, int B, bool PAIRS>
 __global__ void __launch_bounds__(256, HX_LANES_MINB) k_insert_queue(const typename PairTraits<P>::K* __restrict__ keys,
@@ -371,45 +354,7 @@ __global__ void __launch_bounds__(256, HX_LANES_MINB) k_insert_queue(const typen
   fetch();
   unsigned ins = 0, maxd = 0, queued = 0;
   bool fail = false;
-  // One step of the probe of pr, at bucket b; whether it goes on (then from the new b).
-  auto step = [&](const P& pr, uint32_t& b) -> bool {
-    Window<P, B> w;
-    const uint32_t w0 = b & ~(uint32_t)(B - 1);
-    load_buckets<B>(table + w0, w.k, w.v);
-    unsigned match, empty;
-    window_bits<P, B>(w, pr.first, b, match, empty);
-    if (match) {
-      store_value(table + w0 + __ffs(match) - 1, pr.second);
-      return false;
-    }
-    const uint32_t h = home_slot(pr.first, sp);
-    uint32_t to = w0 + B;  // where the probe goes on
-    if (empty) {
-      const unsigned j = __ffs(empty) - 1;
-      K ek = EMPTY;
-      V ev{};
-#pragma unroll
-      for (int t = 0; t < B; ++t)
-        if (t == (int)j) ev = w.v[t];
-      to = w0 + j;
-      if (cas_pair(table + to, ek, ev, pr.first, pr.second)) {
-        ++ins;
-        maxd = max(maxd, ((to - h) & tmask) + 1);
-        return false;
-      }
-      if (ek == pr.first) {
-        store_value(table + to, pr.second);
-        return false;
-      }
-      if (ek != EMPTY) ++to;  // another key took it (else: EMPTY with another value, tried again)
-    }
-    if (((b - h) & tmask) + (to - b) > tmask) {  // round the whole table: no bucket is left
-      fail = true;
-      return false;
-    }
-    b = to & tmask;
-    return true;
-  };
+  auto step = [&](const P& pr, uint32_t& b) { return insert_step<P, B>(table, sp, pr, b, ins, maxd, fail); };
   for (;;) {
     const bool more = __any_sync(0xffffffffu, i < n);
     P pr;
@@ -479,7 +424,6 @@ __global__ void __launch_bounds__(256, HX_LANES_MINB) k_find_queue(const typenam
   __shared__ uint64_t s_i[8][kQueue];  // where its value goes
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  const uint32_t tmask = (1u << sp) - 1u;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   auto fetch = [&]() -> K {
@@ -490,30 +434,19 @@ __global__ void __launch_bounds__(256, HX_LANES_MINB) k_find_queue(const typenam
   K next = fetch();
   unsigned erased = 0, queued = 0;
   auto step = [&](K key, uint64_t at, uint32_t& b) -> bool {
-    Window<P, B> w;
-    const uint32_t w0 = b & ~(uint32_t)(B - 1);
-    load_buckets<B>(table + w0, w.k, w.v);
-    unsigned match, empty;
-    window_bits<P, B>(w, key, b, match, empty);
-    if (match) {
-      const unsigned j = __ffs(match) - 1;
+    uint32_t slot;
+    V v;
+    const int r = find_step<P, B>(table, sp, limit, key, b, slot, v);
+    if (r == FS_HIT) {
       if constexpr (ERASE) {
-        if (cas_key(table + w0 + j, key, PairTraits<P>::TOMB)) ++erased;
+        if (cas_key(table + slot, key, PairTraits<P>::TOMB)) ++erased;
+      } else if constexpr (PAIRS) {
+        pairs[at].second = v;
       } else {
-        V v{};
-#pragma unroll
-        for (int t = 0; t < B; ++t)
-          if (t == (int)j) v = w.v[t];
-        if constexpr (PAIRS) pairs[at].second = v;
-        else vals[at] = v;
+        vals[at] = v;
       }
-      return false;
     }
-    if (empty) return false;
-    // past the longest probe of any key (which is at most the table)
-    const uint32_t d = ((b - home_slot(key, sp)) & tmask) + (w0 + B - b);
-    b = (w0 + B) & tmask;
-    return d < limit;
+    return r == FS_ON;
   };
   for (;;) {
     const bool more = __any_sync(0xffffffffu, i < n);

@@ -539,47 +539,131 @@ __device__ __forceinline__ void insert_one_t1_win(P* tab, int sp, typename PairT
   }
 }
 
-// U keys per thread, elements first + u * stride (those below count), each
-// loaded by load(i, key, val): their first CASes at home are issued together,
-// so U atomics are in flight per thread, and each key is then finished as
-// insert_one_t1 does.
-template <class P, int B, int U, class Load>
-__device__ __forceinline__ void insert_t1_many(P* tab, int sp, unsigned first, unsigned stride, unsigned count,
-                                               const Load& load, unsigned& ins, unsigned& maxd, bool& fail) {
+// ---------------------------------------------------------------------------
+// A probe in single steps of one 32-byte window, for kernels that run the steps of
+// many keys side by side.
+// ---------------------------------------------------------------------------
+// Buckets of the 32-byte window that holds bucket b, from b on: those equal to key, and
+// the EMPTY ones, as bits.
+template <class P, int B>
+__device__ __forceinline__ void window_bits(const Window<P, B>& w, typename PairTraits<P>::K key, uint32_t b,
+                                            unsigned& match, unsigned& empty) {
+  match = empty = 0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    match |= (unsigned)(w.k[j] == key) << j;
+    empty |= (unsigned)(w.k[j] == PairTraits<P>::EMPTY) << j;
+  }
+  const unsigned from = ~0u << (b & (B - 1));
+  match &= from;
+  empty &= from;
+}
+
+// One step of the insert of pr, at bucket b; whether it goes on (then from the new b).
+template <class P, int B>
+__device__ __forceinline__ bool insert_step(P* __restrict__ table, int sp, const P& pr, uint32_t& b, unsigned& ins,
+                                            unsigned& maxd, bool& fail) {
   using K = typename PairTraits<P>::K;
   using V = typename PairTraits<P>::V;
-  K key[U], ek[U];
-  V val[U], ev[U];
-  uint32_t h[U];
-  bool act[U], ok[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const unsigned i = first + u * stride;
-    act[u] = i < count;
-    if (act[u]) {
-      load(i, key[u], val[u]);
-      act[u] = key[u] != PairTraits<P>::EMPTY && key[u] != PairTraits<P>::TOMB;
-    }
+  constexpr K EMPTY = PairTraits<P>::EMPTY;
+  const uint32_t tmask = (1u << sp) - 1u;
+  Window<P, B> w;
+  const uint32_t w0 = b & ~(uint32_t)(B - 1);
+  load_buckets<B>(table + w0, w.k, w.v);
+  unsigned match, empty;
+  window_bits<P, B>(w, pr.first, b, match, empty);
+  if (match) {
+    store_value(table + w0 + __ffs(match) - 1, pr.second);
+    return false;
   }
+  const uint32_t h = home_slot(pr.first, sp);
+  uint32_t to = w0 + B;  // where the probe goes on
+  if (empty) {
+    const unsigned j = __ffs(empty) - 1;
+    K ek = EMPTY;
+    V ev{};
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    ok[u] = false;
-    if (act[u]) {
-      h[u] = home_slot(key[u], sp);
-      ek[u] = PairTraits<P>::EMPTY;
-      ev[u] = 0;
-      ok[u] = cas_pair(tab + h[u], ek[u], ev[u], key[u], val[u]);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    if (!act[u]) continue;
-    if (ok[u]) {
+    for (int t = 0; t < B; ++t)
+      if (t == (int)j) ev = w.v[t];
+    to = w0 + j;
+    if (cas_pair(table + to, ek, ev, pr.first, pr.second)) {
       ++ins;
-      maxd = maxd > 1u ? maxd : 1u;
-    } else {
-      insert_t1_after_cas<P, B>(tab, sp, key[u], val[u], h[u], ek[u], ev[u], ins, maxd, fail);
+      maxd = max(maxd, ((to - h) & tmask) + 1);
+      return false;
     }
+    if (ek == pr.first) {
+      store_value(table + to, pr.second);
+      return false;
+    }
+    if (ek != EMPTY) ++to;  // another key took it (else: EMPTY with another value, tried again)
+  }
+  if (((b - h) & tmask) + (to - b) > tmask) {  // round the whole table: no bucket is left
+    fail = true;
+    return false;
+  }
+  b = to & tmask;
+  return true;
+}
+
+// One step of the look-up of key, at bucket b: found (in bucket slot, with value v), not
+// there, or to go on from the new b. A probe ends after `limit` buckets.
+enum : int { FS_ON = 0, FS_HIT = 1, FS_MISS = 2 };
+template <class P, int B>
+__device__ __forceinline__ int find_step(const P* __restrict__ table, int sp, unsigned limit,
+                                         typename PairTraits<P>::K key, uint32_t& b, uint32_t& slot,
+                                         typename PairTraits<P>::V& v) {
+  const uint32_t tmask = (1u << sp) - 1u;
+  Window<P, B> w;
+  const uint32_t w0 = b & ~(uint32_t)(B - 1);
+  load_buckets<B>(table + w0, w.k, w.v);
+  unsigned match, empty;
+  window_bits<P, B>(w, key, b, match, empty);
+  if (match) {
+    const unsigned j = __ffs(match) - 1;
+    slot = w0 + j;
+#pragma unroll
+    for (int t = 0; t < B; ++t)
+      if (t == (int)j) v = w.v[t];
+    return FS_HIT;
+  }
+  if (empty) return FS_MISS;
+  const uint32_t d = ((b - home_slot(key, sp)) & tmask) + (w0 + B - b);
+  b = (w0 + B) & tmask;
+  return d < limit ? FS_ON : FS_MISS;
+}
+
+// The keys base, base + 1, ... below count of one warp (32 at a time, `stride` apart),
+// those that their first access leaves open waiting in the warp's queue of kQueue
+// entries until 32 of them can take their next step together. first(i, rec) starts key
+// number i and step(rec) takes one step of a key's probe; both say whether it is open.
+constexpr unsigned kQueue = 64;  // fewer than 32 wait while 32 more arrive
+template <class Rec, class First, class Step>
+__device__ __forceinline__ void queue_run(Rec* queue, unsigned base, unsigned stride, unsigned count, int lane,
+                                          const First& first, const Step& step) {
+  const unsigned below = (1u << lane) - 1u;
+  unsigned queued = 0;
+  for (;;) {
+    const bool more = base < count;
+    Rec rec;
+    bool open = false;
+    if (more && queued < 32) {
+      if (base + lane < count) open = first(base + lane, rec);
+      base += stride;
+    } else {
+      if (queued == 0) break;
+      const unsigned take = queued < 32 ? queued : 32;
+      queued -= take;
+      if ((unsigned)lane < take) {
+        rec = queue[queued + lane];
+        open = step(rec);
+        while (open && !more && queued == 0) open = step(rec);  // the last ones: nothing to wait for
+      }
+      __syncwarp();
+    }
+    const unsigned wait = __ballot_sync(0xffffffffu, open);
+    if (open) queue[queued + __popc(wait & below)] = rec;
+    queued += __popc(wait);
+    __syncwarp();
   }
 }
 
