@@ -7,22 +7,31 @@
 // unit; libhx instantiates it for its predicate descriptors.
 //
 // Shape. One cooperative launch of G co-resident CTAs (G = resident CTAs per
-// SM x SMs). The input is cut into slices (one stage of shared memory, 64 KiB
-// by default); phase p gives slice p*G + b to CTA b, so
-// a phase is G consecutive slices. Each CTA keeps STAGES slices in flight,
-// each filled by one bulk copy (cp.async.bulk, completion on an mbarrier).
+// SM x SMs). The input is cut into slices (one stage of shared memory); phase p
+// gives slice p*G + b to CTA b, so a phase is G consecutive slices. Each CTA
+// keeps STAGES slices in flight, each filled by one bulk copy (cp.async.bulk,
+// completion on an mbarrier).
 //   pass 1, phase p: read the slice from shared memory, evaluate the rule (or
 //     sum, for the scan), write the CTA-local result back into the same stage
 //     (the selected elements packed at the front, or the local exclusive
 //     sums), and publish the CTA's count for phase p in a slot of scratch.
-//   pass 2, phase p - D (D phases later): read every CTA's count of that
-//     phase, which by then are almost always published, add up those of the
-//     CTAs before this one and of all earlier phases, write the stage's result
-//     to global memory at that offset, and refill the stage with a later slice.
-// So the input is read once, the output written once, the only exchange
-// between CTAs is one count per CTA per phase, and its latency is hidden
-// behind D phases of work instead of sitting on every tile's critical path
-// as in a decoupled look-back.
+//   pass 2, of an earlier phase: read every CTA's count of that phase, which
+//     by then are almost always published, add up those of the CTAs before
+//     this one and of all earlier phases, write the stage's result to global
+//     memory at that offset, and refill the stage with a later slice.
+// So the input is read once, the output written once, and the only exchange
+// between CTAs is one count per CTA per phase, whose latency is hidden behind
+// other phases instead of sitting on every tile's critical path as in a
+// decoupled look-back.
+//
+// Compaction: two groups of 256 threads select, each from every second slice,
+// and 384 threads write out what they packed. Pass 1 is a chain of dependent
+// steps (load, rule, ranks, barrier, pack) that leaves most issue slots empty:
+// with 16 warps in step the SM issued 1.75 instructions a cycle and DRAM stood
+// at 42%. Two groups fill each other's waits, and the write-out of one phase no
+// longer waits for pass 1 of the next. 2^28 u32, 1 / 25 / 50 / 75 / 99 of 100
+// selected: 304 / 340 / 373 / 419 / 473 us with every thread in both passes,
+// 280 / 305 / 332 / 366 / 420 so. Pairs out of 2^27 buckets: 371 -> 331 us.
 //
 // Co-residency: every CTA waits for the counts of every other, so the launch
 // is cooperative (the runtime guarantees all CTAs resident). Every wait is
@@ -82,6 +91,22 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// A barrier of `threads` threads of the CTA, and the same with an OR over them.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ bool bar_or(int id, int threads, bool p) {
+  unsigned r;
+  asm volatile(
+      "{\n .reg .pred a, b;\n setp.ne.u32 a, %3, 0;\n barrier.cta.red.or.pred b, %1, %2, a;\n selp.u32 %0, 1, 0, b;\n}\n"
+      : "=r"(r)
+      : "r"(id), "r"(threads), "r"((unsigned)p)
+      : "memory");
+  return r != 0;
+}
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -105,54 +130,72 @@ __device__ __forceinline__ unsigned warp_incl_scan(unsigned x, int lane) {
 }
 
 // ---- geometry and scratch -------------------------------------------------
-// Tuned on GB300 over slices of 8-64 KiB, 3-6 stages, deferral 1-3 and
-// 256/512/768/1024-thread blocks (2^28 u32 copy_if and scan).
+// The compaction's. Threads of a CTA: kPack that select, in kGroups groups, and kWrite
+// that write out. 2^28 u32, 1 / 50 / 99 of 100 selected, in us, and pairs of 2^27 buckets:
+//   1 group, 64 KiB slices, 3 stages, D 1, 256 writers   294 / 341 / 407, 351
+//   2 groups, 32 KiB, 6 stages, D 3, 256 writers         268 / 341 / 443, 311
+//   2 groups, 32 KiB, 6 stages, D 3, 384 writers         280 / 332 / 420, 331  (this)
+//   2 groups, 32 KiB, 6 stages, D 1, 256 writers         well behind: a count is published too late
+//   512 writers (64 registers a thread)                  305 / 399 / 447, 360
+//   3 groups of 256, 6 stages                            276 / 353 / 468, 323
 #ifndef HX_STREAM_BLOCK
-#define HX_STREAM_BLOCK 512
+#define HX_STREAM_BLOCK 896
+#endif
+#ifndef HX_STREAM_WRITERS
+#define HX_STREAM_WRITERS 384
+#endif
+#ifndef HX_STREAM_GROUPS
+#define HX_STREAM_GROUPS 2
 #endif
 #ifndef HX_STREAM_R
-#define HX_STREAM_R 8  // uint4 per thread per slice: 512 threads x 8 x 16 B = 64 KiB slices
+#define HX_STREAM_R 8  // uint4 per selecting thread per slice: 256 threads x 8 x 16 B = 32 KiB slices
 #endif
 #ifndef HX_STREAM_STAGES
-#define HX_STREAM_STAGES 3
+#define HX_STREAM_STAGES 6
 #endif
 #ifndef HX_STREAM_DEFER
-#define HX_STREAM_DEFER 1
+#define HX_STREAM_DEFER 3
 #endif
 #ifndef HX_STREAM_LANE_CHUNKS
 #define HX_STREAM_LANE_CHUNKS 0  // compaction: each lane owns kR consecutive uint4s (see the kernel)
 #endif
-#ifndef HX_STREAM_MINB
-#define HX_STREAM_MINB 1  // CTAs per SM the register allocation must allow
-#endif
 constexpr int kBlock = HX_STREAM_BLOCK;
-static_assert(kBlock % 32 == 0 && kBlock <= 1024, "whole warps, at most 32 of them");
+constexpr int kWrite = HX_STREAM_WRITERS;
+constexpr int kPack = kBlock - kWrite;
+constexpr int kGroups = HX_STREAM_GROUPS;
+constexpr int kGroup = kPack / kGroups;  // threads that select from one slice
+constexpr int kWriteBar = 1 + kGroups;   // the writers' barrier; group g has barrier 1 + g, the CTA barrier 0
+static_assert(kWrite % 32 == 0 && kWrite > 0 && kPack % (32 * kGroups) == 0 && kPack > 0 && kBlock <= 1024, "whole warps");
+static_assert(kGroup <= 1024 && kWriteBar < 16, "one barrier per group, one warp scan over a group's warps");
 constexpr int kR = HX_STREAM_R;
 constexpr int kStages = HX_STREAM_STAGES;
 constexpr int kDefer = HX_STREAM_DEFER;
 constexpr bool kLaneChunks = HX_STREAM_LANE_CHUNKS != 0;
+static_assert(kStages % kGroups == 0, "a stage belongs to one group");
 static_assert(kDefer >= 1 && kDefer < kStages, "a stage must be free to load while D phases wait");
-// Count slots per CTA. In phase p a CTA publishes its count of p, then
-// reads every CTA's count of p - D; so when it publishes p it has read every
-// count of p - 1 - D, every CTA has published p - 1 - D, and every CTA has
-// therefore read every count of the phases up to p - 2 - 2D. The row of
-// phase p is the row of phase p - kSlots, so kSlots = 2D + 2.
+// Count slots per CTA. A CTA publishes its count of phase p once its own writers are
+// done with p - 1 - D, for which they read every CTA's count of that phase; so every
+// CTA has published p - 1 - D, and every CTA's writers are done with p - 2 - 2D. The
+// row of phase p is the row of phase p - kSlots, so kSlots = 2D + 2.
 constexpr int kSlots = 2 * kDefer + 2;
-constexpr int kMaxGrid = 1024;  // CTAs at most (GB300: 152 SMs x 1-2 CTAs); a larger device runs 1024
-constexpr int kSlotLoads = (kMaxGrid + kBlock - 1) / kBlock;  // count slots each thread reads per phase
-constexpr unsigned kSliceBytes = kBlock * kR * 16;
+constexpr int kMaxGrid = 512;  // CTAs at most (GB300: 152); a larger device runs 512
+constexpr int kSlotLoads = (kMaxGrid + kWrite - 1) / kWrite;  // count slots each writer reads per phase
+constexpr unsigned kSliceBytes = kGroup * kR * 16;
 
-// Scratch: [error word u32][pad .. 256 B][count slots u64 x kSlots x grid].
-// The launcher zeroes the part it uses.
-constexpr uint64_t kScratchBytes = 256 + 8ull * kSlots * kMaxGrid;
-inline uint64_t scratch_bytes_used(unsigned grid) { return 256 + 8ull * kSlots * grid; }
-// Scratch a pass over n elements of elem_bytes each needs: its grid is at
-// most one CTA per slice.
+// Scratch: [error word u32][pad .. 256 B][count slots u64, rows of one per CTA].
+// The launcher zeroes the part it uses: one row per phase, at most kSlots.
+// 32 B per 64 KiB of input, for at most 1024 of those, hold the scan's 4 rows of one
+// slot per 64 KiB slice. They hold the compaction's rows too: one row of 8 B per 32 KiB
+// slice when there is one phase, and when there are P > 1 on G CTAs, min(P, 8) rows of
+// G slots, against more than (P - 1) G slices.
+constexpr uint64_t kScratchBytes = 256 + 32ull * 1024;
+static_assert(8ull * kSlots * kMaxGrid <= 32ull * 1024, "the compaction's slots fit");
+// Scratch a pass over n elements of elem_bytes each needs.
 inline uint64_t scratch_need(uint64_t n, unsigned elem_bytes) {
-  uint64_t slices = (n * elem_bytes + kSliceBytes - 1) / kSliceBytes;
-  if (slices < 1) slices = 1;
-  if (slices > (uint64_t)kMaxGrid) slices = kMaxGrid;
-  return scratch_bytes_used((unsigned)slices);
+  uint64_t units = (n * elem_bytes + 65535) / 65536;
+  if (units < 1) units = 1;
+  if (units > 1024) units = 1024;
+  return 256 + 32 * units;
 }
 
 struct Scratch {
@@ -204,86 +247,53 @@ struct Done {                              // what the pass reports, and where i
 };
 
 // ---------------------------------------------------------------------------
-// The kernel. SCAN: T = O = uint32_t, out[i] = sum of in[0..i) mod 2^32.
-// Otherwise: out[0..c) = the selected elements (projected to O) in input
+// The compaction: out[0..c) = the selected elements (projected to O) in input
 // order, writes beyond `capacity` dropped, c to *done.d_count.
 // ---------------------------------------------------------------------------
-template <class T, class O, class Sel, bool SCAN>
-__global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __restrict__ in, O* __restrict__ out, uint64_t n,
-                                                  Sel sel, uint64_t capacity, Done done, Scratch sc) {
+template <class T, class O, class Sel>
+__global__ void __launch_bounds__(kBlock, 1) k_compact(const T* __restrict__ in, O* __restrict__ out, uint64_t n, Sel sel,
+                                                     uint64_t capacity, Done done, Scratch sc) {
   constexpr int E = 16 / sizeof(T);
-  constexpr int WARPS = kBlock / 32;
-  constexpr unsigned SU4 = kBlock * kR;  // uint4 per slice
-  constexpr unsigned SE = SU4 * E;       // elements per slice
-  static_assert(!SCAN || std::is_same<T, uint32_t>::value, "the scan is over uint32_t");
+  constexpr int WARPS = kGroup / 32, WWARPS = kWrite / 32;
+  constexpr unsigned SU4 = kGroup * kR;  // uint4 per slice
+  constexpr unsigned SE = SU4 * E;      // elements per slice
   static_assert(sizeof(O) <= sizeof(T), "the packed result fits in its stage");
   extern __shared__ __align__(128) uint4 s_stage[];  // kStages x SU4
-  __shared__ __align__(8) uint64_t s_bar[kStages];
-  __shared__ unsigned s_warp[WARPS];
+  __shared__ __align__(8) uint64_t s_full[kStages];     // the stage holds its slice
+  __shared__ __align__(8) uint64_t s_packed[kStages];   // the stage holds its packed result
+  __shared__ __align__(8) uint64_t s_written[kStages];  // the stage's result is written out
+  __shared__ unsigned s_warp[kGroups][2][WARPS];  // by the parity of the group's phases
   __shared__ unsigned s_cnt[kStages];
-  __shared__ uint2 s_red[WARPS];  // per warp: (count before this CTA, phase total), both < 2^32
-  __shared__ int s_abort;
+  __shared__ uint2 s_red[WWARPS];  // per warp: (count before this CTA, phase total), both < 2^32
 
   // Device-side inputs: the same values for every CTA, so every CTA runs the
   // same phases and none waits on a CTA that skipped.
   if (done.n_from && *done.n_from < n) n = *done.n_from;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const unsigned G = gridDim.x, b = blockIdx.x;
   const uint64_t full_slices = n / SE;  // slices wholly inside [0, n)
   const unsigned phases = (unsigned)(((n + SE - 1) / SE + G - 1) / G);  // below 2^32 - kDefer (launch)
-  unsigned pend = 0;                    // thread 0: stages with a bulk copy not yet seen complete
-  unsigned par = 0;                     // parity of the next wait, bit per stage
-
-  // Fill stage st with the slice of phase p (thread 0): a whole slice by one
-  // bulk copy; the ragged last slice and slices past n are read later with
-  // plain loads, so their barrier phase completes with no bytes.
-  auto issue = [&](int st, unsigned p) {
-    const uint64_t t = (uint64_t)p * G + b;
-    if (t < full_slices) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the stage come first
-      mbar_expect_tx(&s_bar[st], kSliceBytes);
-      bulk_load(s_stage + (size_t)st * SU4, in + t * SE, kSliceBytes, &s_bar[st]);
-    } else {
-      mbar_expect_tx(&s_bar[st], 0);
-    }
-    pend |= 1u << st;
-  };
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) mbar_init(&s_bar[s], 1);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&s_packed[s], WARPS);
+      mbar_init(&s_written[s], 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    s_abort = 0;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int s = 0; s < kStages && (unsigned)s < phases; ++s) issue(s, s);
-
-  // result count (or sum) of the phases already written, after any elements placed before this pass
-  unsigned long long base = done.base_from ? *done.base_from : 0ull;
-  bool failed = false;
-  // stage and count-slot row of phase p (pass 1) and of phase p - kDefer
-  // (pass 2), advanced by one each phase instead of computed by division
-  unsigned st1 = 0, st2 = 0, sl1 = 0, sl2 = 0;
   auto next = [](unsigned& i, unsigned m) { i = i + 1 == m ? 0u : i + 1; };
-  for (unsigned p = 0; p < phases + kDefer; ++p) {
-    // The count slots that pass 2 reads below were published kDefer phases
-    // ago: load them now, so that their latency overlaps pass 1.
-    unsigned long long pv[kSlotLoads];
-    if (p >= (unsigned)kDefer) {
-      const unsigned long long* row = sc.slots + sl2 * G;
-#pragma unroll
-      for (int k = 0; k < kSlotLoads; ++k) {
-        const unsigned c = threadIdx.x + k * kBlock;
-        pv[k] = c < G ? ld_relaxed(row + c) : 0ull;
-      }
-    }
-    // ---- pass 1: phase p -------------------------------------------------
-    if (p < phases) {
-      const unsigned st = st1;
-      const bool ok = mbar_wait(&s_bar[st], (par >> st) & 1u);
-      if (ok) {  // a failed wait leaves par and pend as they were, for the drain below
-        par ^= 1u << st;
-        pend &= ~(1u << st);
-      }
+
+  if (threadIdx.x < kPack) {
+    // ---- a selecting group: pass 1 of every kGroups-th phase --------------------
+    const unsigned grp = threadIdx.x / kGroup;
+    const int warp = (threadIdx.x % kGroup) >> 5;
+    unsigned st = grp;    // stage of phase p
+    unsigned par = 0;     // parity of the next wait for a full stage, bit per stage
+    unsigned buf = 0;
+    for (unsigned p = grp; p < phases; p += kGroups) {
+      const bool ok = mbar_wait(&s_full[st], (par >> st) & 1u);
+      par ^= 1u << st;
       const uint64_t t = (uint64_t)p * G + b;
       const bool whole = t < full_slices;
       const uint64_t e0 = t * SE;
@@ -296,7 +306,7 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
       // part and row r holds its uint4 (r + l) mod kR: rotated, so that with
       // kR = 8 the 8 lanes of a shared-memory wavefront read 8 different bank
       // groups.
-      constexpr bool LANE = kLaneChunks && !SCAN && (kR & (kR - 1)) == 0 && kR * E <= 32;
+      constexpr bool LANE = kLaneChunks && (kR & (kR - 1)) == 0 && kR * E <= 32;
       auto u_of = [&](int r) -> unsigned {
         if constexpr (LANE) return wbase + lane * kR + ((r + lane) & (kR - 1));
         else return wbase + r * 32 + lane;
@@ -316,10 +326,6 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
           }
         }
       }
-      if (__syncthreads_or(!ok)) {  // stage st is read; a failed wait stops every thread here
-        failed = true;
-        break;
-      }
       unsigned pre[kR];
       unsigned acc = 0;
       unsigned bits[kR];
@@ -327,11 +333,7 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
       unsigned lm = 0;  // lane chunks: the lane's selections, bit j*E + q for element q of its uint4 j
 #pragma unroll
       for (int r = 0; r < kR; ++r) {
-        unsigned c;
-        if constexpr (SCAN) {
-          c = x[r][0] + x[r][1] + x[r][2] + x[r][3];
-          bits[r] = 0;
-        } else {
+        {
           const uint64_t e = e0 + (uint64_t)u_of(r) * E;
           unsigned m = 0;
           if (whole) {  // block-uniform: no per-element bounds checks in a whole slice
@@ -356,13 +358,7 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
           }
           bits[r] = m;
           if constexpr (LANE) lm |= m << (((r + lane) & (kR - 1)) * E);
-          c = __popc(m);
-        }
-        cnt[r] = c;
-        if constexpr (SCAN) {
-          const unsigned incl = warp_incl_scan(c, lane);
-          pre[r] = acc + incl - c;
-          acc += __shfl_sync(0xffffffffu, incl, 31);
+          cnt[r] = __popc(m);
         }
       }
       unsigned lane_pre = 0;  // lane chunks: selections of the warp's lanes before this one
@@ -371,7 +367,7 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
         const unsigned incl = warp_incl_scan(c, lane);
         lane_pre = incl - c;
         acc = __shfl_sync(0xffffffffu, incl, 31);
-      } else if constexpr (!SCAN) {
+      } else {
         // Ranks of the selections: a lane's count per uint4 is at most 4 and a
         // warp's sum at most 128, so four uint4s share one 32-bit word as byte
         // lanes with no carries between them: one warp scan per four uint4s.
@@ -393,28 +389,31 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
           acc += (tot_w[r / 4] >> (8 * (r % 4))) & 0xffu;
         }
       }
-      if (lane == 0) s_warp[warp] = acc;
-      __syncthreads();
-      if (warp == 0) {
-        const unsigned wt = lane < WARPS ? s_warp[lane] : 0u;
-        const unsigned wincl = warp_incl_scan(wt, lane);
-        if (lane < WARPS) s_warp[lane] = wincl - wt;
-        if (lane == 31) {
-          s_cnt[st] = wincl;
-          // publish this CTA's count (or sum, mod 2^32) of phase p, tagged with p + 1
-          st_relaxed(sc.slots + sl1 * G + b, ((unsigned long long)(p + 1) << 32) | wincl);
-        }
+      if (lane == 0) s_warp[grp][buf][warp] = acc;
+      // The one barrier of a phase: the group has read the stage, and has its warps' counts.
+      if (bar_or(1 + grp, kGroup, !ok)) {  // a failed wait stops the whole group here
+        if (lane == 0) atomicExch(sc.error, 1u);
+        return;
       }
-      __syncthreads();
-      // the CTA-local result, in place in the stage (every thread has read it)
-      const unsigned woff = s_warp[warp];
-      if constexpr (SCAN) {
-#pragma unroll
-        for (int r = 0; r < kR; ++r) {
-          const unsigned o0 = woff + pre[r], o1 = o0 + x[r][0], o2 = o1 + x[r][1], o3 = o2 + x[r][2];
-          stage[wbase + r * 32 + lane] = make_uint4(o0, o1, o2, o3);
+      const unsigned wt = lane < WARPS ? s_warp[grp][buf][lane] : 0u;
+      const unsigned wincl = warp_incl_scan(wt, lane);
+      const unsigned woff = __shfl_sync(0xffffffffu, wincl - wt, warp);
+      buf ^= 1u;
+      if (warp == 0 && lane == 31) {
+        s_cnt[st] = wincl;
+        // the row's last readers are done (kSlots); if that wait runs out, the writers' waits do too
+        if (p > (unsigned)kDefer) {
+          const unsigned w = p - 1 - kDefer;
+          mbar_wait(&s_written[w % kStages], (w / kStages) & 1u);
         }
-      } else {
+        // publish this CTA's count of phase p, tagged with p + 1
+        st_relaxed(sc.slots + (p % kSlots) * G + b, ((unsigned long long)(p + 1) << 32) | wincl);
+      }
+      // Packing starts together, also for the lane above: without this barrier a 2^28-element
+      // copy_if is 3-10% slower (446 -> 497 us at 99 of 100 selected, one group).
+      bar_sync(1 + grp, kGroup);
+      // the CTA-local result, in place in the stage (every thread has read it)
+      {
         O* packed = reinterpret_cast<O*>(stage);
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
@@ -431,18 +430,285 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
             if (bits[r] & (1u << q)) packed[o++] = hxs::project<T, O>(x[r][q]);
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_packed[st]);
+      st += kGroups;
+      if (st >= (unsigned)kStages) st -= kStages;
+    }
+    return;
+  }
+
+  // ---- the writing warps: loads ahead, pass 2 of one phase after the other ------
+  const unsigned tid = threadIdx.x - kPack;
+  const int warp = tid >> 5;
+  unsigned issued[kStages];  // thread 0 of them: loads issued per stage
+#pragma unroll
+  for (int s = 0; s < kStages; ++s) issued[s] = 0;
+  // Fill stage st with the slice of phase p: a whole slice by one bulk copy; the
+  // ragged last slice and slices past n are read later with plain loads, so their
+  // barrier phase completes with no bytes.
+  auto issue = [&](unsigned st, unsigned p) {
+    const uint64_t t = (uint64_t)p * G + b;
+    if (t < full_slices) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the stage come first
+      mbar_expect_tx(&s_full[st], kSliceBytes);
+      bulk_load(s_stage + (size_t)st * SU4, in + t * SE, kSliceBytes, &s_full[st]);
+    } else {
+      mbar_expect_tx(&s_full[st], 0);
+    }
+#pragma unroll
+    for (int s = 0; s < kStages; ++s) issued[s] += (unsigned)(s == (int)st);
+  };
+  if (tid == 0)
+    for (unsigned s = 0; s < (unsigned)kStages && s < phases; ++s) issue(s, s);
+  // result count of the phases already written, after any elements placed before this pass
+  unsigned long long base = done.base_from ? *done.base_from : 0ull;
+  bool failed = false;
+  unsigned st = 0, sl = 0, par = 0;
+  unsigned long long pv[kSlotLoads];  // the counts of phase q, read ahead while phase q - 1 is written
+#pragma unroll
+  for (int k = 0; k < kSlotLoads; ++k) pv[k] = 0;  // no phase's tag: read when the wait is over
+  for (unsigned q = 0; q < phases; ++q) {
+    // Every CTA's count of phase q: the sum over CTAs before this one, and
+    // the total. A phase holds at most kMaxGrid slices of at most 2^14
+    // elements, so both fit 32 bits.
+    const unsigned long long* row = sc.slots + sl * G;
+    bool ok = mbar_wait(&s_packed[st], (par >> st) & 1u);
+    par ^= 1u << st;
+    unsigned before = 0, total = 0;
+#pragma unroll
+    for (int k = 0; k < kSlotLoads; ++k) {
+      const unsigned c = tid + k * kWrite;
+      if (c >= G) break;
+      unsigned long long v = pv[k];
+      if (ok && (unsigned)(v >> 32) != q + 1) v = ld_relaxed(row + c);
+      if (ok && (unsigned)(v >> 32) != q + 1) {
+        const unsigned long long t0 = globaltimer();
+        unsigned i = 0;
+        while ((unsigned)(v >> 32) != q + 1) {
+          if ((++i & 63) == 0) {
+            if (ld_relaxed_u32(sc.error) || globaltimer() - t0 > kWaitNs) {
+              ok = false;
+              break;
+            }
+            __nanosleep(64);
+          }
+          v = ld_relaxed(row + c);
+        }
+      }
+      const unsigned cnt = (unsigned)v;
+      total += cnt;
+      if (c < b) before += cnt;
+    }
+    // only the warps that read a slot reduce; the others hold zeros
+    const unsigned nw = G >= (unsigned)kWrite ? (unsigned)WWARPS : (G + 31) / 32;
+    if ((unsigned)warp < nw) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+      }
+      if (lane == 0) s_red[warp] = make_uint2(before, total);
+    }
+    if (bar_or(kWriteBar, kWrite, !ok)) {
+      failed = true;
+      break;
+    }
+    next(sl, kSlots);
+    if (q + 1 < phases) {
+      const unsigned long long* ahead = sc.slots + sl * G;
+#pragma unroll
+      for (int k = 0; k < kSlotLoads; ++k) {
+        const unsigned c = tid + k * kWrite;
+        if (c < G) pv[k] = ld_relaxed(ahead + c);
+      }
+    }
+    before = 0;
+    total = 0;
+    for (unsigned w = 0; w < nw; ++w) {
+      const uint2 r = s_red[w];
+      before += r.x;
+      total += r.y;
+    }
+    const unsigned long long prefix = base + before;
+    const uint4* stage = s_stage + (size_t)st * SU4;
+    {
+      const O* packed = reinterpret_cast<const O*>(stage);
+      unsigned cnt = s_cnt[st];
+      if (prefix >= capacity) cnt = 0;
+      else if (capacity - prefix < cnt) cnt = (unsigned)(capacity - prefix);
+      O* to = out + prefix;
+#pragma unroll 8
+      for (unsigned i = tid; i < cnt; i += kWrite) to[i] = packed[i];
+    }
+    base += total;
+    bar_sync(kWriteBar, kWrite);  // stage st is written out, s_red is read
+    if (tid == 0) {
+      mbar_arrive(&s_written[st]);
+      if (q + kStages < phases) issue(st, q + kStages);
+    }
+    next(st, kStages);
+  }
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(sc.error, 1u);
+      // no copy is issued after a failure: give each one still in flight a
+      // bounded wait before the CTA exits
+#pragma unroll
+      for (int s = 0; s < kStages; ++s)
+        if (issued[s]) mbar_wait(&s_full[s], (issued[s] - 1) & 1u);
+    }
+    return;
+  }
+  if (b == 0 && tid == 0) {
+    if (done.d_count) *done.d_count = base < done.count_max ? base : done.count_max;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The scan: out[i] = sum of in[0..i) mod 2^32. The same phases, with every
+// thread in both passes: it writes as much as it reads and is bound by memory,
+// and the split of the compaction below costs it more than it saves (2^28 - 57
+// elements, 342 us; with selecting groups and writers apart 347-380 us).
+// ---------------------------------------------------------------------------
+namespace scan {
+constexpr int kR = 8, kStages = 3, kDefer = 1, kSlots = 2 * kDefer + 2;
+constexpr unsigned kSliceBytes = 512 * kR * 16;
+constexpr int kMaxGrid = 1024;
+constexpr int kSlotLoads = (kMaxGrid + 511) / 512;  // count slots each thread reads per phase
+}  // namespace scan
+template <int kBlock = 512>  // a template only so that every unit that includes this may define it
+__global__ void __launch_bounds__(kBlock, 1) k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                                                    uint64_t n, Scratch sc) {
+  constexpr int E = 4;
+  constexpr int WARPS = kBlock / 32;
+  constexpr unsigned SU4 = kBlock * scan::kR;  // uint4 per slice
+  constexpr unsigned SE = SU4 * E;       // elements per slice
+  extern __shared__ __align__(128) uint4 s_stage[];  // scan::kStages x SU4
+  __shared__ __align__(8) uint64_t s_bar[scan::kStages];
+  __shared__ unsigned s_warp[WARPS];
+  __shared__ uint2 s_red[WARPS];  // per warp: (count before this CTA, phase total), both < 2^32
+  __shared__ int s_abort;
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned G = gridDim.x, b = blockIdx.x;
+  const uint64_t full_slices = n / SE;  // slices wholly inside [0, n)
+  const unsigned phases = (unsigned)(((n + SE - 1) / SE + G - 1) / G);  // below 2^32 - scan::kDefer (launch)
+  unsigned pend = 0;                    // thread 0: stages with a bulk copy not yet seen complete
+  unsigned par = 0;                     // parity of the next wait, bit per stage
+
+  // Fill stage st with the slice of phase p (thread 0): a whole slice by one
+  // bulk copy; the ragged last slice and slices past n are read later with
+  // plain loads, so their barrier phase completes with no bytes.
+  auto issue = [&](int st, unsigned p) {
+    const uint64_t t = (uint64_t)p * G + b;
+    if (t < full_slices) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the stage come first
+      mbar_expect_tx(&s_bar[st], scan::kSliceBytes);
+      bulk_load(s_stage + (size_t)st * SU4, in + t * SE, scan::kSliceBytes, &s_bar[st]);
+    } else {
+      mbar_expect_tx(&s_bar[st], 0);
+    }
+    pend |= 1u << st;
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < scan::kStages; ++s) mbar_init(&s_bar[s], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_abort = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int s = 0; s < scan::kStages && (unsigned)s < phases; ++s) issue(s, s);
+
+  unsigned long long base = 0;  // sum of the phases already written
+  bool failed = false;
+  // stage and count-slot row of phase p (pass 1) and of phase p - scan::kDefer
+  // (pass 2), advanced by one each phase instead of computed by division
+  unsigned st1 = 0, st2 = 0, sl1 = 0, sl2 = 0;
+  auto next = [](unsigned& i, unsigned m) { i = i + 1 == m ? 0u : i + 1; };
+  for (unsigned p = 0; p < phases + scan::kDefer; ++p) {
+    // The count slots that pass 2 reads below were published scan::kDefer phases
+    // ago: load them now, so that their latency overlaps pass 1.
+    unsigned long long pv[scan::kSlotLoads];
+    if (p >= (unsigned)scan::kDefer) {
+      const unsigned long long* row = sc.slots + sl2 * G;
+#pragma unroll
+      for (int k = 0; k < scan::kSlotLoads; ++k) {
+        const unsigned c = threadIdx.x + k * kBlock;
+        pv[k] = c < G ? ld_relaxed(row + c) : 0ull;
+      }
+    }
+    // ---- pass 1: phase p -------------------------------------------------
+    if (p < phases) {
+      const unsigned st = st1;
+      const bool ok = mbar_wait(&s_bar[st], (par >> st) & 1u);
+      if (ok) {  // a failed wait leaves par and pend as they were, for the drain below
+        par ^= 1u << st;
+        pend &= ~(1u << st);
+      }
+      const uint64_t t = (uint64_t)p * G + b;
+      const bool whole = t < full_slices;
+      const uint64_t e0 = t * SE;
+      uint32_t x[scan::kR][E];
+      uint4* stage = s_stage + (size_t)st * SU4;
+      const unsigned wbase = warp * 32 * scan::kR;  // this warp's first uint4 of the slice
+#pragma unroll
+      for (int r = 0; r < scan::kR; ++r) {
+        const unsigned u = wbase + r * 32 + lane;
+        if (whole) {
+          const uint4 q = stage[u];
+          memcpy(&x[r][0], &q, 16);
+        } else {
+#pragma unroll
+          for (int q = 0; q < E; ++q) {
+            const uint64_t e = e0 + (uint64_t)u * E + q;
+            if (e < n) x[r][q] = in[e];
+            else x[r][q] = 0;
+          }
+        }
+      }
+      if (__syncthreads_or(!ok)) {  // stage st is read; a failed wait stops every thread here
+        failed = true;
+        break;
+      }
+      unsigned pre[scan::kR];
+      unsigned acc = 0;
+#pragma unroll
+      for (int r = 0; r < scan::kR; ++r) {
+        const unsigned c = x[r][0] + x[r][1] + x[r][2] + x[r][3];
+        const unsigned incl = warp_incl_scan(c, lane);
+        pre[r] = acc + incl - c;
+        acc += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) s_warp[warp] = acc;
+      __syncthreads();
+      if (warp == 0) {
+        const unsigned wt = lane < WARPS ? s_warp[lane] : 0u;
+        const unsigned wincl = warp_incl_scan(wt, lane);
+        if (lane < WARPS) s_warp[lane] = wincl - wt;
+        if (lane == 31) {
+          // publish this CTA's sum of phase p (mod 2^32), tagged with p + 1
+          st_relaxed(sc.slots + sl1 * G + b, ((unsigned long long)(p + 1) << 32) | wincl);
+        }
+      }
+      __syncthreads();
+      // the CTA-local result, in place in the stage (every thread has read it)
+      const unsigned woff = s_warp[warp];
+#pragma unroll
+      for (int r = 0; r < scan::kR; ++r) {
+        const unsigned o0 = woff + pre[r], o1 = o0 + x[r][0], o2 = o1 + x[r][1], o3 = o2 + x[r][2];
+        stage[wbase + r * 32 + lane] = make_uint4(o0, o1, o2, o3);
+      }
     }
     // ---- pass 2: phase p - D ---------------------------------------------
-    if (p >= (unsigned)kDefer) {
-      const unsigned q = p - kDefer;
+    if (p >= (unsigned)scan::kDefer) {
+      const unsigned q = p - scan::kDefer;
       const unsigned st = st2;
-      // Every CTA's count of phase q: the sum over CTAs before this one, and
-      // the total. A phase holds at most kMaxGrid slices of at most 2^14
-      // elements, so both fit 32 bits (the scan's sums are taken mod 2^32).
+      // Every CTA's sum of phase q, mod 2^32: of the CTAs before this one, and of all.
       unsigned before = 0, total = 0;
       bool ok = true;
 #pragma unroll
-      for (int k = 0; k < kSlotLoads; ++k) {
+      for (int k = 0; k < scan::kSlotLoads; ++k) {
         const unsigned c = threadIdx.x + k * kBlock;
         if (c >= G) break;
         const unsigned long long* slot = sc.slots + sl2 * G + c;
@@ -490,61 +756,44 @@ __global__ void __launch_bounds__(kBlock, HX_STREAM_MINB) k_stream(const T* __re
       const unsigned long long prefix = base + before;
       const uint4* stage = s_stage + (size_t)st * SU4;
       const uint64_t t = (uint64_t)q * G + b;
-      if constexpr (SCAN) {
-        const uint64_t e0 = t * SE;
-        const unsigned add = (unsigned)prefix;
-        const bool whole = t < full_slices;
-        uint32_t* o32 = reinterpret_cast<uint32_t*>(out);
-        for (unsigned u = threadIdx.x; u < SU4; u += kBlock) {
-          const uint4 v = stage[u];
-          const uint4 w = make_uint4(v.x + add, v.y + add, v.z + add, v.w + add);
-          const uint64_t e = e0 + (uint64_t)u * 4;
-          if (whole) {
-            __stcs(reinterpret_cast<uint4*>(o32 + e), w);
-          } else {
-            const unsigned a[4] = {w.x, w.y, w.z, w.w};
+      const uint64_t e0 = t * SE;
+      const unsigned add = (unsigned)prefix;
+      const bool whole = t < full_slices;
+      for (unsigned u = threadIdx.x; u < SU4; u += kBlock) {
+        const uint4 v = stage[u];
+        const uint4 w = make_uint4(v.x + add, v.y + add, v.z + add, v.w + add);
+        const uint64_t e = e0 + (uint64_t)u * 4;
+        if (whole) {
+          __stcs(reinterpret_cast<uint4*>(out + e), w);
+        } else {
+          const unsigned a[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (e + k < n) o32[e + k] = a[k];
-          }
-        }
-      } else {
-        const O* packed = reinterpret_cast<const O*>(stage);
-        const unsigned cnt = s_cnt[st];
-        for (unsigned i = threadIdx.x; i < cnt; i += kBlock) {
-          const unsigned long long dst = prefix + i;
-          if (dst < capacity) out[dst] = packed[i];
+          for (int k = 0; k < 4; ++k)
+            if (e + k < n) out[e + k] = a[k];
         }
       }
       base += total;
       __syncthreads();  // stage st is written out
-      if (threadIdx.x == 0 && q + kStages < phases) issue(st, q + kStages);
-      next(st2, kStages);
-      next(sl2, kSlots);
+      if (threadIdx.x == 0 && q + scan::kStages < phases) issue(st, q + scan::kStages);
+      next(st2, scan::kStages);
+      next(sl2, scan::kSlots);
     }
-    next(st1, kStages);
-    next(sl1, kSlots);
+    next(st1, scan::kStages);
+    next(sl1, scan::kSlots);
   }
   if (failed) {
     if (threadIdx.x == 0) {
       atomicExch(sc.error, 1u);
       // no copy is issued after a failure: give each one still in flight a
       // bounded wait before the CTA exits
-      for (int s = 0; s < kStages; ++s)
+      for (int s = 0; s < scan::kStages; ++s)
         if ((pend >> s) & 1u) mbar_wait(&s_bar[s], (par >> s) & 1u);
     }
-    return;
-  }
-  if (b == 0 && threadIdx.x == 0) {
-    if (done.d_count) *done.d_count = base < done.count_max ? base : done.count_max;
   }
 }
-
 // ---- host side -------------------------------------------------------------
-inline size_t smem_bytes() { return (size_t)kStages * kSliceBytes; }
-
 // Co-resident CTAs of one kernel on the current device (SMs x CTAs per SM,
-// at most kMaxGrid), with the kernel's shared-memory limit raised first.
+// at most max_grid), with the kernel's shared-memory limit raised first.
 // The limit is raised on every call (cheap, and it survives a device reset
 // that would drop it); the occupancy query runs once per kernel and device.
 // The cache is keyed by the kernel's host-side address, not by its template
@@ -553,8 +802,7 @@ inline size_t smem_bytes() { return (size_t)kStages * kSliceBytes; }
 // function in each, while a static of an inline function is one object
 // shared by all of them.
 template <class Kern>
-inline cudaError_t resident_grid(Kern kern, unsigned* grid) {
-  const size_t smem = smem_bytes();
+inline cudaError_t resident_grid(Kern kern, int block, size_t smem, int max_grid, unsigned* grid) {
   cudaError_t e = cudaSuccess;
   if (smem > 48 * 1024) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -574,17 +822,44 @@ inline cudaError_t resident_grid(Kern kern, unsigned* grid) {
     }
   }
   int per_sm = 0, sms = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem)) != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   long g = (long)per_sm * sms;
   if (g < 1) return cudaErrorInvalidConfiguration;
-  if (g > kMaxGrid) g = kMaxGrid;
+  if (g > max_grid) g = max_grid;
   {
     std::lock_guard<std::mutex> lk(mu);
     cache[key] = (unsigned)g;
   }
   *grid = (unsigned)g;
   return cudaSuccess;
+}
+
+// Launches `kern`, one CTA of `block` threads per slice and at most as many as are
+// resident together, with `rows` rows of count slots (fewer if there are fewer phases)
+// and the error word zeroed first, on the stream.
+template <class Kern, class... Args>
+inline cudaError_t launch_phases(Kern kern, int block, size_t smem, int max_grid, uint64_t slices, unsigned rows,
+                                 void* scratch, cudaStream_t s, Args... args) {
+  unsigned grid = 0;
+  cudaError_t e = resident_grid(kern, block, smem, max_grid, &grid);
+  if (e != cudaSuccess) return e;
+  if (slices < grid) grid = (unsigned)slices;
+  if (slices / grid >= 0xffff0000ull) return cudaErrorInvalidValue;  // phases are counted in 32 bits
+  const uint64_t phases = (slices + grid - 1) / grid;
+  e = cudaMemsetAsync(scratch, 0, 256 + 8ull * (phases < rows ? phases : rows) * grid, s);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args..., carve(scratch));
 }
 
 // Launches one pass over n > 0 elements of a 16-byte-aligned `in` (and, for
@@ -594,27 +869,15 @@ inline cudaError_t resident_grid(Kern kern, unsigned* grid) {
 template <class T, class O, class Sel, bool SCAN>
 inline cudaError_t launch(const T* in, O* out, uint64_t n, const Sel& sel, uint64_t capacity, Done done,
                           void* scratch, cudaStream_t s) {
-  auto kern = k_stream<T, O, Sel, SCAN>;
-  unsigned grid = 0;
-  cudaError_t e = resident_grid(kern, &grid);
-  if (e != cudaSuccess) return e;
-  constexpr uint64_t SE = (uint64_t)kBlock * kR * (16 / sizeof(T));
-  const uint64_t slices = (n + SE - 1) / SE;
-  if (slices < grid) grid = (unsigned)slices;
-  if (slices / grid >= 0xffff0000ull) return cudaErrorInvalidValue;  // phases are counted in 32 bits
-  e = cudaMemsetAsync(scratch, 0, scratch_bytes_used(grid), s);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kBlock);
-  cfg.dynamicSmemBytes = smem_bytes();
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, in, out, n, sel, capacity, done, carve(scratch));
+  if constexpr (SCAN) {
+    constexpr uint64_t SE = scan::kSliceBytes / 4;
+    return launch_phases(k_scan<512>, 512, (size_t)scan::kStages * scan::kSliceBytes, scan::kMaxGrid,
+                         (n + SE - 1) / SE, scan::kSlots, scratch, s, in, out, n);
+  } else {
+    constexpr uint64_t SE = kSliceBytes / sizeof(T);
+    return launch_phases(k_compact<T, O, Sel>, kBlock, (size_t)kStages * kSliceBytes, kMaxGrid, (n + SE - 1) / SE,
+                         kSlots, scratch, s, in, out, n, sel, capacity, done);
+  }
 }
 
 }  // namespace hxs
