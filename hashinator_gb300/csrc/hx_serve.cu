@@ -324,6 +324,7 @@ struct Slot {
   GrowTask* d_tasks = nullptr;
   GrowChunk* d_chunks = nullptr;
   size_t chunk_cap = 0;
+  uint64_t tile_cap = 0;
 };
 
 }  // namespace hx
@@ -335,7 +336,6 @@ struct hx_server {
   uint32_t max_maps = 0;
   uint32_t max_round_requests = 0;
   uint64_t max_round_keys = 0;
-  uint32_t tile_keys = 4096;
   std::vector<hx::ServeMap> maps;
   hx::SMap* d_maps = nullptr;
   hx::DInfo* d_info = nullptr;
@@ -377,6 +377,40 @@ static void view_of(hx_server* sv, unsigned i, hx_map* v) {
 #define HX_SERVE_LONG_PROBE 64
 #endif
 constexpr unsigned kLongProbe = HX_SERVE_LONG_PROBE;
+
+// Tile size: one key per thread. A request is a link in its map's chain of stages, and
+// the chain is as long as its tiles take: with 4096 keys a tile (16 keys per thread,
+// one after the other, each a probe through the tombstones that erases leave) a round
+// of 2048 requests on 256 maps, 3.1 M keys, took 1.2 ms on fresh tables and 7.1 ms
+// after 5 - 40 such rounds; with 1024 keys 1.1 / 3.7 ms, 512 1.1 / 2.8 ms, 256 1.1 /
+// 1.8 ms. Very large rounds take two keys per thread: a tile costs some 3 us of its
+// own, and a fresh round of 23 M keys 2.5 ms with 256, 2.2 ms with 512 keys.
+constexpr uint64_t kTileKeys = 256;
+static uint64_t round_tile(uint64_t round_keys) { return round_keys < (1ull << 23) ? kTileKeys : 2 * kTileKeys; }
+
+// Room for the tiles of a round. A request above the round's limit of keys runs alone,
+// however large it is, so a slot's buffers grow when such a request comes. The slot is
+// free: nothing on the device reads them.
+static hx_status round_tiles(Slot& sl, const std::vector<Pending>& round, uint64_t tile) {
+  uint64_t need = 0;
+  for (const Pending& p : round) need += std::max<uint64_t>(1, (p.r.n + tile - 1) / tile);
+  if (need <= sl.tile_cap) return HX_OK;
+  if (need > 0xFFFFFFFFull) return HX_ERR_INVALID_ARG;
+  STile *h = nullptr, *d = nullptr;
+  cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&h), need * sizeof(STile));
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d), need * sizeof(STile));
+  if (e != cudaSuccess) {
+    if (h) cudaFreeHost(h);
+    cudaGetLastError();
+    return cuda_status(e);
+  }
+  cudaFreeHost(sl.h_tiles);
+  cudaFree(sl.d_tiles);
+  sl.h_tiles = h;
+  sl.d_tiles = d;
+  sl.tile_cap = need;
+  return HX_OK;
+}
 
 // Completed rounds: completion times, fill bounds refreshed from the
 // round's metadata snapshot.
@@ -443,7 +477,8 @@ hx_status hx_server_create(hx_server** out, int key_bytes, uint64_t memory_budge
   sv->max_maps = max_maps;
   sv->max_round_requests = max_round_requests;
   sv->max_round_keys = max_round_keys;
-  const uint64_t max_tiles = max_round_requests + max_round_keys / 256 + 1;
+  // tiles of a round within max_round_keys; a larger request takes a round of its own (round_tiles)
+  const uint64_t max_tiles = max_round_requests + max_round_keys / kTileKeys + 1;
   cudaError_t e = cudaStreamCreateWithFlags(&sv->s, cudaStreamNonBlocking);
   // Tables grow and shrink through the stream-ordered allocator, from a pool
   // of the server's own: freed tables stay in it (release threshold = max)
@@ -477,6 +512,7 @@ hx_status hx_server_create(hx_server** out, int key_bytes, uint64_t memory_budge
     if (e == cudaSuccess)
       e = cudaMalloc(reinterpret_cast<void**>(&sl.d_cnt), (2 + max_round_requests) * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDefault);
+    sl.tile_cap = max_tiles;
     sl.chunk_cap = 1 << 16;
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&sl.h_tasks), max_maps * sizeof(GrowTask));
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&sl.h_chunks), sl.chunk_cap * sizeof(GrowChunk));
@@ -602,6 +638,11 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
     keys += p.r.n;
     round.push_back(p);
     sv->queue.pop_front();
+  }
+  const uint64_t tile = round_tile(keys);
+  if ((st = round_tiles(*sl, round, tile)) != HX_OK) {
+    sv->queue.insert(sv->queue.begin(), round.begin(), round.end());  // they wait for the next step
+    return st;
   }
   // Table maintenance and admission of inserts, in admission order. Insert
   // never reuses TOMBSTONE buckets (kernels_NVIDIA.h:383-407), so a map whose
@@ -762,14 +803,6 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
   if (nreq == 0) return HX_OK;
   std::stable_sort(order.begin(), order.end(),
                    [](const std::pair<int, unsigned>& a, const std::pair<int, unsigned>& b) { return a.first < b.first; });
-  // Tile size: one key per thread. A request is a link in its map's chain of stages, and
-  // the chain is as long as its tiles take: with 4096 keys a tile (16 keys per thread,
-  // one after the other, each a probe through the tombstones that erases leave) a round
-  // of 2048 requests on 256 maps, 3.1 M keys, took 1.2 ms on fresh tables and 7.1 ms
-  // after 5 - 40 such rounds; with 1024 keys 1.1 / 3.7 ms, 512 1.1 / 2.8 ms, 256 1.1 /
-  // 1.8 ms. Very large rounds take two keys per thread: a tile costs some 3 us of its
-  // own, and a fresh round of 23 M keys 2.5 ms with 256, 2.2 ms with 512 keys.
-  const uint64_t tile = round_keys < (1ull << 23) ? 256 : 512;
   const unsigned nstages = (unsigned)stage_depth.size();
   for (unsigned j = 0; j < nstages; ++j) sl->h_rem[j] = 0;
   unsigned ntiles = 0;
