@@ -293,7 +293,7 @@ struct ServeMap {
   uint64_t in_flight = 0;        // inserts launched in rounds not yet completed
   uint64_t in_flight_erase = 0;  // erase keys launched in rounds not yet completed
   uint64_t rehash_round = 0;     // first round that runs on the current table
-  unsigned base_probe = 0;       // longest probe of the first snapshot of the current table (0: none yet)
+  unsigned base_probe = 0;       // longest probe that its keys alone gave the current table (0: no snapshot yet)
   bool tangled = false;          // its probes run long through tombstones
 };
 
@@ -370,9 +370,11 @@ static void view_of(hx_server* sv, unsigned i, hx_map* v) {
 // and a probe to such a home passes all of them, long before the table is full: rounds
 // that insert and erase the same keys took 1.1 ms at first and 7 ms after 200 rounds
 // (256 maps, 3.1 M keys; with this rule 1.1 ms, with a bound of 128 or 256 buckets 1.1 /
-// 1.2 ms). A map whose longest probe passed
-// kLongProbe buckets and twice what it was on the fresh table, with tombstones enough to
-// account for it, is rehashed at its size before its next round, which drops them.
+// 1.2 ms). A map whose longest probe passed kLongProbe buckets and twice what its keys
+// alone gave it, with tombstones enough to account for it, is rehashed at its size before
+// its next insert, which drops them. Before an insert only: a caller that looks up or
+// erases may hold the address of the table. It is done for speed alone, so it is left for
+// a later round where the budget has no room for the second copy or the allocation fails.
 #ifndef HX_SERVE_LONG_PROBE
 #define HX_SERVE_LONG_PROBE 64
 #endif
@@ -444,8 +446,9 @@ static hx_status reap(hx_server* sv, bool wait_oldest) {
       if (sl.round_no >= m.rehash_round) {
         m.tomb_ub = sl.h_info[i].tombstones + m.in_flight_erase;
         const unsigned probe = sl.h_info[i].max_probe;
-        if (m.base_probe == 0) m.base_probe = probe;
-        m.tangled = probe > kLongProbe && probe > 2 * m.base_probe && sl.h_info[i].tombstones * 4 > probe;
+        const bool accounts = sl.h_info[i].tombstones * 4 > probe;
+        if (m.base_probe == 0 || (!accounts && probe > m.base_probe)) m.base_probe = probe;
+        m.tangled = probe > kLongProbe && probe > 2 * m.base_probe && accounts;
       }
     }
     sl.busy = false;
@@ -655,20 +658,28 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
   std::vector<GrowTask> tasks;
   std::vector<void*> old_tables;
   const uint64_t this_round = sv->rounds;
+  std::vector<std::pair<uint32_t, ServeMap>> before;  // the maps as they were
+  const uint64_t used_before = sv->used;
+  const hx_server_stats st_before = sv->st;
   // One batched rehash per map and round: a second need in the same round replaces
-  // the pending target with the larger table.
-  auto schedule = [&](uint32_t map, int nsp) -> hx_status {
+  // the pending target with the larger table. Nothing changes if the table cannot be had.
+  auto schedule = [&](uint32_t map, int nsp) -> cudaError_t {
     ServeMap& m = sv->maps[map];
     const uint64_t nbytes = (1ull << nsp) * pb(sv);
     int& slot_of = grow_of[map];
     void* nt = nullptr;
-    HX_CUDA(cudaMallocFromPoolAsync(&nt, nbytes, sv->pool, sv->s));
+    const cudaError_t e = cudaMallocFromPoolAsync(&nt, nbytes, sv->pool, sv->s);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return e;
+    }
     if (slot_of < 0) {
       slot_of = (int)tasks.size();
       tasks.push_back(GrowTask{m.table, nt, 1ull << m.sp, nsp, map});
       old_tables.push_back(m.table);
+      before.push_back({map, m});
     } else {
-      HX_CUDA(cudaFreeAsync(tasks[slot_of].new_table, sv->s));  // never used
+      cudaFreeAsync(tasks[slot_of].new_table, sv->s);  // never used
       tasks[slot_of].new_table = nt;
       tasks[slot_of].new_sp = nsp;
     }
@@ -682,12 +693,21 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
     m.tangled = false;
     m.base_probe = 0;
     m.rehash_round = this_round;
-    return HX_OK;
+    return cudaSuccess;
   };
+  // Until the rehashes are launched, the round can be undone: its requests wait for the next step.
+  auto undo = [&](hx_status e) -> hx_status {
+    for (const GrowTask& t : tasks) cudaFreeAsync(t.new_table, sv->s);
+    for (auto& b : before) sv->maps[b.first] = b.second;
+    sv->used = used_before;
+    sv->st = st_before;
+    sv->queue.insert(sv->queue.begin(), round.begin(), round.end());
+    return e;
+  };
+  uint64_t second_copies = 0;  // bytes of the rehashes for speed, whose old tables are counted in `used`
   for (size_t i = 0; i < round.size(); ++i) {
     const hx_request& r = round[i].r;
     ServeMap& m = sv->maps[r.map];
-    if (m.tangled && r.n && (st = schedule(r.map, m.sp)) != HX_OK) return st;
     if (r.op == SOP_ERASE) {
       era[r.map] += r.n;
       continue;
@@ -705,7 +725,16 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
         admitted[i] = 0;  // cannot make room within the budget: reject this insert
         continue;
       }
-      if ((st = schedule(r.map, nsp)) != HX_OK) return st;
+      const cudaError_t e = schedule(r.map, nsp);
+      if (e == cudaErrorMemoryAllocation) {
+        admitted[i] = 0;  // the device has no room
+        continue;
+      }
+      if (e != cudaSuccess) return undo(cuda_status(e));
+    } else if (m.tangled && sv->used + second_copies + m.bytes <= sv->budget) {
+      const cudaError_t e = schedule(r.map, m.sp);
+      if (e == cudaSuccess) second_copies += m.bytes;
+      else m.tangled = false, m.base_probe *= 2;  // tried again when its probes have doubled
     }
     add[r.map] += r.n;
   }
@@ -723,13 +752,21 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
       for (uint64_t a0 = 0; a0 < tasks[i].old_n; a0 += kChunk)
         movec.push_back(GrowChunk{i, (unsigned)std::min<uint64_t>(kChunk, tasks[i].old_n - a0), a0});
     }
-    if (fillc.size() + movec.size() > sl->chunk_cap) {
-      cudaStreamSynchronize(sv->s);  // rare: grow the staging buffers
+    if (fillc.size() + movec.size() > sl->chunk_cap) {  // rare: grow the staging buffers
+      const size_t cap = (fillc.size() + movec.size()) * 2;
+      GrowChunk *h = nullptr, *d = nullptr;
+      cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&h), cap * sizeof(GrowChunk));
+      if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&d), cap * sizeof(GrowChunk));
+      if (e != cudaSuccess) {
+        if (h) cudaFreeHost(h);
+        cudaGetLastError();
+        return undo(cuda_status(e));
+      }
       cudaFreeHost(sl->h_chunks);
       cudaFree(sl->d_chunks);
-      sl->chunk_cap = (fillc.size() + movec.size()) * 2;
-      HX_CUDA(cudaMallocHost(reinterpret_cast<void**>(&sl->h_chunks), sl->chunk_cap * sizeof(GrowChunk)));
-      HX_CUDA(cudaMalloc(reinterpret_cast<void**>(&sl->d_chunks), sl->chunk_cap * sizeof(GrowChunk)));
+      sl->h_chunks = h;
+      sl->d_chunks = d;
+      sl->chunk_cap = cap;
     }
     std::copy(tasks.begin(), tasks.end(), sl->h_tasks);
     std::copy(fillc.begin(), fillc.end(), sl->h_chunks);
@@ -762,6 +799,7 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
   uint64_t round_keys = 0;
   sl->tags.clear();
   sl->inserts.clear();
+  sl->erases.clear();
   for (size_t i = 0; i < round.size(); ++i) {
     const hx_request& r = round[i].r;
     if (!admitted[i]) {

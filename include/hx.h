@@ -366,7 +366,12 @@ hx_status hx_batch_inject_stall(hx_batch_plan* plan, uint32_t map, int phase, in
  * next round while the GPU runs the current one). Before a round, a map
  * whose load factor would pass max_load_factor is grown by an on-device
  * rehash; tables are admitted against memory_budget_bytes, and an insert
- * that cannot grow its table within the budget completes with HX_ERR_OOM.
+ * that cannot grow its table within the budget, or within what the device
+ * has left, completes with HX_ERR_OOM. A map whose probes run long through
+ * tombstones is rehashed at its size before an insert, where the budget has
+ * room for the second copy. So a table (hx_server_bucket_data) may move in a
+ * round that inserts into its map, and in no other. A request of more than
+ * max_round_keys keys runs as a round of its own.
  * One host thread drives a server. Tables live in a stream-ordered memory
  * pool that the server creates for itself, with its release threshold at
  * the maximum, so that growth does not return memory to the driver at every

@@ -16,6 +16,7 @@ namespace {
 struct Block {
   void* base;
   size_t mapped, bytes;
+  bool host;
 };
 std::map<void*, Block> g_live;
 struct Pool {
@@ -28,14 +29,14 @@ bool g_capturing = false;
 cudaError_t g_last = cudaSuccess;
 
 cudaError_t fail(cudaError_t e) { return g_last = e; }
-cudaError_t make(void** p, size_t bytes) {
+cudaError_t make(void** p, size_t bytes, bool host = false) {
   const size_t page = 4096, body = (bytes + page - 1) / page * page + (bytes ? 0 : page);
   char* m = static_cast<char*>(mmap(nullptr, body + page, PROT_READ | PROT_WRITE,
                                     MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0));
   if (m == MAP_FAILED) return fail(cudaErrorMemoryAllocation);
   mprotect(m + body, page, PROT_NONE);
   *p = m + (body - (bytes + 15) / 16 * 16);
-  g_live[*p] = Block{m, body + page, bytes};
+  g_live[*p] = Block{m, body + page, bytes, host};
   return cudaSuccess;
 }
 cudaError_t drop(void* p) {
@@ -66,9 +67,9 @@ cudaStream_t g_stream;
 }  // namespace
 
 extern "C" {
-void* fake_find(size_t bytes) {  // a live allocation of exactly so many bytes
+void* fake_find(size_t bytes) {  // a live device allocation of exactly so many bytes
   for (auto& b : g_live)
-    if (b.second.bytes == bytes) return b.first;
+    if (b.second.bytes == bytes && !b.second.host) return b.first;
   return nullptr;
 }
 void fake_fail_pool_from(size_t bytes) { g_fail_from = bytes; }
@@ -111,7 +112,7 @@ cudaError_t cudaMallocHost(void** p, size_t n) {
     --g_fail_host;
     return fail(cudaErrorMemoryAllocation);
   }
-  return make(p, n);
+  return make(p, n, true);
 }
 cudaError_t cudaFree(void* p) { return drop(p); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return drop(p); }
