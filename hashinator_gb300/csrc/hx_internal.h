@@ -32,6 +32,7 @@ struct hx_map {
   hx::Tuning tune;
   bool err_success = false;  // info->err is known to be success (see set_err_success)
   bool viewed = false;       // a device view was handed out: kernels of the caller may write info->err
+  bool replayed = false;     // an insert, clean or resize was captured: replays may change fill and info->err unseen
   std::mutex mu;  // guards scratch growth; a map is not thread-safe otherwise
 };
 

@@ -992,12 +992,18 @@ static hx_status try_bulk(const hx_map* m, BulkOp op, const void* keys, const vo
                   s, done);
 }
 
+// A call under capture runs again with every replay of its graph, which the host does
+// not see: from then on it takes nothing for known that such a replay may change.
+static void note_capture(hx_map* m, cudaStream_t s) {
+  if (!m->replayed && capturing(s)) m->replayed = true;
+}
+
 // err = success before an insert (hashers.h:50), unless the device word is known to
-// hold it: after a clear, until a kernel that may set fail, a peek_status or a device
-// view (whose kernels write it unseen). A call under capture writes it always, as its
-// replays follow other work than the capture did.
+// hold it: after a clear, until a kernel that may set fail, a peek_status, a device
+// view (whose kernels write it unseen) or a captured call (whose replays do).
 static hx_status set_err_success(hx_map* m, cudaStream_t s) {
-  if (m->err_success && !capturing(s)) return HX_OK;
+  note_capture(m, s);
+  if (m->err_success && !m->replayed) return HX_OK;
   HX_CUDA(cudaMemsetAsync(&m->info->err, 0, sizeof(int), s));
   return HX_OK;
 }
@@ -1218,6 +1224,7 @@ hx_status hx_clean_tombstones(hx_map* m, hx_stream stream) {
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::lock_guard<std::mutex> g(m->mu);
+  note_capture(m, s);
   return is_p32(m) ? launch_clean<P32>(m, s) : launch_clean<P64>(m, s);
 }
 
@@ -1236,6 +1243,7 @@ hx_status hx_extract_keys(hx_map* m, const hx_pred* pred, void* d_out_keys, uint
 hx_status hx_resize(hx_map* m, int new_size_power, hx_stream stream) {
   HX_RANGE("hx_resize");
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
+  note_capture(m, static_cast<cudaStream_t>(stream));
   return rehash(m, new_size_power, static_cast<cudaStream_t>(stream));
 }
 

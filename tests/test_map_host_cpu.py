@@ -1,0 +1,30 @@
+"""A map's host-side bookkeeping without a GPU (host_runtime.py): what a replay of a
+captured call changes on the device is not taken for known."""
+from host_runtime import run_on_host
+
+INFO = """
+class DInfo(ctypes.Structure):
+    _fields_ = [("fill", ctypes.c_uint64), ("tombstones", ctypes.c_uint64), ("max_probe", ctypes.c_uint32),
+                ("err", ctypes.c_int32)]
+def dinfo():
+    return DInfo.from_address(lib.fake_find(72))
+FAIL = hx.STATUS_FAIL
+"""
+
+
+def test_status_after_a_replay_between_clear_and_insert(tmp_path):
+    run_on_host(tmp_path, INFO + """
+m = hx.Hashmap(10, 4)
+d = dinfo()
+for captured in (False, True):
+    if captured:
+        lib.fake_capture(1)
+        m.insert(KEYS, KEYS, n=100, target_lf=0.0)
+        lib.fake_capture(0)
+    m.clear()
+    d.err = 0            # what the clear kernel leaves
+    if captured:
+        d.err = FAIL     # what a replay that fills the table leaves
+    m.insert(KEYS, KEYS, n=10, target_lf=0.0)
+    assert d.err == 0, (captured, d.err)
+""")
