@@ -370,8 +370,7 @@ struct hx_batch {
   unsigned long long* d_off = nullptr;
   int* d_sp = nullptr;
   hx::DInfo* d_info = nullptr;
-  void* scratch = nullptr;  // per-map plain clean_tombstones scratch (shared)
-  uint64_t scratch_bytes = 0;
+  hx::ScratchBuf scratch;  // per-map plain clean_tombstones scratch (shared)
 };
 
 struct hx_batch_plan {
@@ -576,8 +575,7 @@ static void make_view(hx_batch* b, unsigned i, hx_map* v) {
   v->buckets = static_cast<char*>(b->arena) + b->off[i] * pbytes(b);
   v->info = b->d_info + i;
   v->fill_ub = b->fill_ub[i];
-  v->scratch = b->scratch;
-  v->scratch_bytes = b->scratch_bytes;
+  v->scratch = &b->scratch;
 }
 
 }  // namespace hx
@@ -648,7 +646,7 @@ hx_status hx_batch_destroy(hx_batch* b) {
   cudaFree(b->d_off);
   cudaFree(b->d_sp);
   cudaFree(b->d_info);
-  cudaFree(b->scratch);
+  b->scratch.release();
   delete b;
   pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);
@@ -921,8 +919,6 @@ hx_status hx_batch_run_per_map(hx_batch_plan* p, hx_stream stream) {
       if (st != HX_OK) return st;
     }
     b->fill_ub[i] = v.fill_ub;
-    b->scratch = v.scratch;  // the views share one clean scratch buffer
-    b->scratch_bytes = v.scratch_bytes;
   }
   return HX_OK;
 }

@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdint>
 #include <mutex>
+#include <vector>
 #include <cuda_runtime.h>
 #include "../../include/hx.h"
 #include "hx_probe.cuh"
@@ -17,6 +18,21 @@ struct Tuning {
   bool wide = false;  // thread-per-key windows of 64 B instead of 32 B
 };
 
+// A device buffer kept from call to call. One that a graph was captured with lives on
+// when a larger one takes its place: replays use it.
+struct ScratchBuf {
+  void* ptr = nullptr;
+  uint64_t bytes = 0;
+  bool in_graph = false;
+  std::vector<void*> kept;
+  void release() {  // after a device synchronisation
+    if (ptr) cudaFree(ptr);
+    for (void* p : kept) cudaFree(p);
+    ptr = nullptr;
+    bytes = 0;
+    kept.clear();
+  }
+};
 
 }  // namespace hx
 
@@ -27,8 +43,8 @@ struct hx_map {
   void* buckets = nullptr;
   hx::DInfo* info = nullptr;
   uint64_t fill_ub = 0;  // host upper bound on fill (exact after a sync)
-  void* scratch = nullptr;
-  uint64_t scratch_bytes = 0;
+  hx::ScratchBuf own_scratch;
+  hx::ScratchBuf* scratch = &own_scratch;  // views of a batch's maps share the batch's
   hx::Tuning tune;
   bool err_success = false;  // info->err is known to be success (see set_err_success)
   bool viewed = false;       // a device view was handed out: kernels of the caller may write info->err

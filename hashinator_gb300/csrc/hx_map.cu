@@ -858,7 +858,43 @@ static hx_status launch_find(hx_map* m, const void* keys, void* vals, void* pair
   return after_launch();
 }
 
-static hx_status ensure_scratch(hx_map* m, uint64_t bytes, cudaStream_t s);
+// The map's scratch for one call. In a capture, where the map's buffer cannot be
+// replaced, a larger need is met by memory of the graph's own.
+class MapScratch {
+ public:
+  void* ptr = nullptr;
+  hx_status get(hx_map* m, uint64_t bytes, cudaStream_t stream) {
+    ScratchBuf& b = *m->scratch;
+    const bool captured = capturing(stream);
+    if (b.bytes < bytes) {
+      if (captured) {
+        HX_CUDA(cudaMallocAsync(&ptr, bytes, stream));
+        s = stream;
+        graphs = true;
+        return HX_OK;
+      }
+      if (b.ptr && b.in_graph) b.kept.push_back(b.ptr);
+      else if (b.ptr) HX_CUDA(cudaFreeAsync(b.ptr, stream));
+      b.ptr = nullptr;
+      b.bytes = 0;
+      b.in_graph = false;
+      uint64_t n = 1;
+      while (n < bytes) n <<= 1;
+      HX_CUDA(pool_alloc(&b.ptr, n, stream));
+      b.bytes = n;
+    }
+    b.in_graph |= captured;
+    ptr = b.ptr;
+    return HX_OK;
+  }
+  ~MapScratch() {
+    if (graphs) cudaFreeAsync(ptr, s);
+  }
+
+ private:
+  cudaStream_t s = nullptr;
+  bool graphs = false;
+};
 
 // clean_tombstones: the pass over the slices, then, if there can be any, the keys
 // that it listed (their count stays on the device).
@@ -869,20 +905,21 @@ static hx_status launch_clean(hx_map* m, cudaStream_t s) {
   const unsigned grid = (unsigned)(n / slots);
   P* table = static_cast<P*>(m->buckets);
   uint64_t cap = 0;
+  MapScratch list;
   hx_status st;
   if (grid > 1) {
     cap = m->fill_ub < n ? m->fill_ub : n;  // listed keys <= fill <= fill_ub
-    if ((st = ensure_scratch(m, (cap + 1) * sizeof(P), s)) != HX_OK) return st;
+    if ((st = list.get(m, (cap + 1) * sizeof(P), s)) != HX_OK) return st;
   }
   constexpr int PER = 32 / sizeof(P);
   auto launch = [&](auto kern) -> hx_status {
     const size_t smem = clean_smem<P>(slots);
     if (smem > 32 * 1024) HX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kCleanThreads, smem, s>>>(table, slots, m->sp, m->info, static_cast<P*>(m->scratch), cap);
+    kern<<<grid, kCleanThreads, smem, s>>>(table, slots, m->sp, m->info, static_cast<P*>(list.ptr), cap);
     return after_launch();
   };
   if ((st = slots >= PER ? launch(k_clean<P, PER>) : launch(k_clean<P, 1>)) != HX_OK || grid == 1) return st;
-  return launch_insert<P>(m, nullptr, nullptr, m->scratch, cap, &m->info->left, s);
+  return launch_insert<P>(m, nullptr, nullptr, list.ptr, cap, &m->info->left, s);
 }
 
 template <class P>
@@ -898,18 +935,6 @@ static hx_status fill_empty(hx_map* m, void* t, uint64_t n, cudaStream_t s) {
     return HX_ERR_INVALID_ARG;
   }
   return is_p32(m) ? launch_fill_empty<P32>(t, n, m->info, s) : launch_fill_empty<P64>(t, n, m->info, s);
-}
-
-static hx_status ensure_scratch(hx_map* m, uint64_t bytes, cudaStream_t s) {
-  if (m->scratch_bytes >= bytes) return HX_OK;
-  if (m->scratch) HX_CUDA(cudaFreeAsync(m->scratch, s));
-  m->scratch = nullptr;
-  m->scratch_bytes = 0;
-  uint64_t b = 1;
-  while (b < bytes) b <<= 1;
-  HX_CUDA(pool_alloc(&m->scratch, b, s));
-  m->scratch_bytes = b;
-  return HX_OK;
 }
 
 static hx_status read_info(hx_map* m, DInfo* out, cudaStream_t s) {
@@ -1046,22 +1071,23 @@ static hx_status extract(hx_map* m, const hx_pred* pred, void* d_out, uint64_t c
   const bool p32 = is_p32(m);
   const uint64_t need = p32 ? compact_scratch_need<P32>(n) : compact_scratch_need<P64>(n);
   const uint64_t sc_bytes = (need + 255) / 256 * 256;
-  hx_status st = ensure_scratch(m, sc_bytes + 256, s);
+  MapScratch sc;
+  hx_status st = sc.get(m, sc_bytes + 256, s);
   if (st != HX_OK) return st;
   unsigned long long* cnt = d_count ? reinterpret_cast<unsigned long long*>(d_count)
-                                    : reinterpret_cast<unsigned long long*>(static_cast<char*>(m->scratch) + sc_bytes);
+                                    : reinterpret_cast<unsigned long long*>(static_cast<char*>(sc.ptr) + sc_bytes);
   cudaError_t e;
   bool sk = false;
   if (p32) {
     using O = typename std::conditional<KEYS, uint32_t, P32>::type;
     e = launch_compact<P32, O>(static_cast<const P32*>(m->buckets), static_cast<O*>(d_out), n, *pred,
                                       TableRef<P32>{static_cast<const P32*>(m->buckets), m->sp}, capacity, cnt,
-                                      m->scratch, s, &sk);
+                                      sc.ptr, s, &sk);
   } else {
     using O = typename std::conditional<KEYS, uint64_t, P64>::type;
     e = launch_compact<P64, O>(static_cast<const P64*>(m->buckets), static_cast<O*>(d_out), n, *pred,
                                       TableRef<P64>{static_cast<const P64*>(m->buckets), m->sp}, capacity, cnt,
-                                      m->scratch, s, &sk);
+                                      sc.ptr, s, &sk);
   }
   if (e != cudaSuccess) return cuda_status(e);
   if ((st = after_launch()) != HX_OK) return st;
@@ -1069,7 +1095,7 @@ static hx_status extract(hx_map* m, const hx_pred* pred, void* d_out, uint64_t c
     unsigned long long c = 0;
     unsigned int err = 0;
     HX_CUDA(cudaMemcpyAsync(&c, cnt, sizeof(c), cudaMemcpyDeviceToHost, s));
-    HX_CUDA(cudaMemcpyAsync(&err, scan_error_word(m->scratch, sk), sizeof(err), cudaMemcpyDeviceToHost, s));
+    HX_CUDA(cudaMemcpyAsync(&err, scan_error_word(sc.ptr, sk), sizeof(err), cudaMemcpyDeviceToHost, s));
     HX_CUDA(cudaStreamSynchronize(s));
     *h_count = c;
     if (err) return HX_ERR_TIMEOUT;
@@ -1119,7 +1145,7 @@ hx_status hx_map_destroy(hx_map* m) {
   cudaError_t e = cudaDeviceSynchronize();
   if (m->buckets) cudaFree(m->buckets);
   if (m->info) cudaFree(m->info);
-  if (m->scratch) cudaFree(m->scratch);
+  m->own_scratch.release();
   delete m;
   pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);

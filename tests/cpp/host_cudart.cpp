@@ -16,7 +16,7 @@ namespace {
 struct Block {
   void* base;
   size_t mapped, bytes;
-  bool host;
+  bool host, captured;
 };
 std::map<void*, Block> g_live;
 struct Pool {
@@ -36,7 +36,7 @@ cudaError_t make(void** p, size_t bytes, bool host = false) {
   if (m == MAP_FAILED) return fail(cudaErrorMemoryAllocation);
   mprotect(m + body, page, PROT_NONE);
   *p = m + (body - (bytes + 15) / 16 * 16);
-  g_live[*p] = Block{m, body + page, bytes, host};
+  g_live[*p] = Block{m, body + page, bytes, host, g_capturing};
   return cudaSuccess;
 }
 cudaError_t drop(void* p) {
@@ -71,6 +71,11 @@ void* fake_find(size_t bytes) {  // a live device allocation of exactly so many 
   for (auto& b : g_live)
     if (b.second.bytes == bytes && !b.second.host) return b.first;
   return nullptr;
+}
+int fake_live(int captured) {  // live device allocations: made under capture, or outside
+  int n = 0;
+  for (auto& b : g_live) n += !b.second.host && b.second.captured == (captured != 0);
+  return n;
 }
 void fake_fail_pool_from(size_t bytes) { g_fail_from = bytes; }
 void fake_fail_host(int count) { g_fail_host = count; }

@@ -28,3 +28,29 @@ for captured in (False, True):
     m.insert(KEYS, KEYS, n=10, target_lf=0.0)
     assert d.err == 0, (captured, d.err)
 """)
+
+
+def test_scratch_of_captured_calls(tmp_path):
+    run_on_host(tmp_path, INFO + """
+lib.fake_live.argtypes = [ctypes.c_int]
+pred, count = hx.Pred.value_even().c(), 1 << 12
+mem = ctypes.c_uint64()
+def extract(m):  # with the count left on the device
+    assert lib.hx_extract_pattern(m._m, ctypes.byref(pred), KEYS, 100, ctypes.addressof(mem), None, None) == 0
+m = hx.Hashmap(20, 4)
+lib.fake_capture(1)
+extract(m)
+m.insert(KEYS, KEYS, n=1 << 18, target_lf=0.0)
+m.clean_tombstones()
+lib.fake_capture(0)
+assert lib.fake_live(1) == 0  # the map keeps nothing that belongs to the graph
+extract(m)                    # takes a buffer of the map's own
+lib.fake_capture(1)
+extract(m)                    # replays use that buffer
+lib.fake_capture(0)
+held = lib.fake_live(0)
+m.clean_tombstones()          # takes a larger one: the graph's lives on
+assert lib.fake_live(0) == held + 1 and lib.fake_live(1) == 0
+m.close()
+assert lib.fake_live(0) == 0
+""")

@@ -45,3 +45,43 @@ def test_status_after_a_replay_that_filled_the_table(hx, w):
     m.insert(dk[at:at + 1], dv[at:at + 1], target_lf=0.0, stream=s)  # a key that is there: it succeeds
     assert m.peek_status(stream=s) == hx.STATUS_SUCCESS
     m.close()
+
+
+@pytest.mark.parametrize("w", [4, 8])
+def test_a_captured_clean_brings_its_own_scratch(hx, w):
+    import torch
+    sp, n = 15, 20001
+    k, v = workloads.distinct_keys(n, w, 4), workloads.values(n, w, 4)
+    dk, dv = _dev(k), _dev(v)
+    gone = dk[: n // 4].contiguous()
+    out = torch.empty_like(dv)
+    fill = int(np.array(FILL, _dt(w)).view(np.int32 if w == 4 else np.int64))
+    s = torch.cuda.Stream()
+    m = hx.Hashmap(sp, w, stream=s)
+    m.insert(dk, dv, target_lf=0.0, stream=s)  # sizes the launch; the map has no scratch yet
+    torch.cuda.synchronize()
+
+    def work():
+        out.fill_(fill)
+        m.clear(stream=s)
+        m.insert(dk, dv, target_lf=0.0, stream=s)
+        m.erase(gone, stream=s)
+        m.clean_tombstones(stream=s)
+        m.retrieve(dk, out, stream=s)
+
+    g = _captured(s, work)
+    want = v.copy()
+    want[: n // 4] = FILL
+    for _ in range(3):
+        out.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(_host(out, w), want)
+        with torch.cuda.stream(s):
+            m.clean_tombstones(stream=s)  # eager calls in between use the map's own
+            assert m.extract_all_keys(torch.empty(n, dtype=dk.dtype, device="cuda"), stream=s) == n - n // 4
+        inf = m.info(stream=s)
+        assert (inf.fill, inf.tombstone_counter, inf.err) == (n - n // 4, 0, hx.STATUS_SUCCESS)
+    del g
+    m.close()
