@@ -576,6 +576,7 @@ static void make_view(hx_batch* b, unsigned i, hx_map* v) {
   v->info = b->d_info + i;
   v->fill_ub = b->fill_ub[i];
   v->scratch = &b->scratch;
+  v->replayed = true;  // plans may run in graphs of the caller's, past fill_ub
 }
 
 }  // namespace hx

@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(kCleanThreads, 3) k_clean(P* table, unsigned s
   if (tid == 0) {
     const unsigned n = aways + s_over;
     s_left0 = n ? atomicAdd(&info->left_next, (unsigned long long)n) : 0ull;
+    if (s_left0 + n > left_cap) atomicExch(&info->err, HX_STATUS_FAIL);  // more keys than fill says: some are lost
     s_over = 0;
   }
   // ---- write back ----------------------------------------------------------

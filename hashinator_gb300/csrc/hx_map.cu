@@ -908,9 +908,12 @@ static hx_status launch_clean(hx_map* m, cudaStream_t s) {
   MapScratch list;
   hx_status st;
   if (grid > 1) {
-    cap = m->fill_ub < n ? m->fill_ub : n;  // listed keys <= fill <= fill_ub
-    if ((st = list.get(m, (cap + 1) * sizeof(P), s)) != HX_OK) return st;
+    // Listed keys <= fill, and fill <= fill_ub unless replays or a caller's kernels insert
+    // unseen: then there is room for every bucket.
+    cap = m->fill_ub < n && !m->replayed && !m->viewed ? m->fill_ub : n;
+    if ((st = list.get(m, cap * sizeof(P), s)) != HX_OK) return st;
   }
+  m->err_success = false;  // the kernels may set fail
   constexpr int PER = 32 / sizeof(P);
   auto launch = [&](auto kern) -> hx_status {
     const size_t smem = clean_smem<P>(slots);

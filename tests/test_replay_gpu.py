@@ -85,3 +85,37 @@ def test_a_captured_clean_brings_its_own_scratch(hx, w):
         assert (inf.fill, inf.tombstone_counter, inf.err) == (n - n // 4, 0, hx.STATUS_SUCCESS)
     del g
     m.close()
+
+
+@pytest.mark.parametrize("w", [4, 8])
+def test_clean_after_a_replay_keeps_every_key(hx, w):
+    import torch
+    sp = 15  # several slices: keys whose run crosses a slice's end go through the list
+    n = int(0.9 * (1 << sp))
+    k, v = workloads.distinct_keys(n, w, 5), workloads.values(n, w, 5)
+    dk, dv = _dev(k), _dev(v)
+    gone = dk[: n // 3].contiguous()
+    s = torch.cuda.Stream()
+    m = hx.Hashmap(sp, w, stream=s)
+    m.insert(dk, dv, target_lf=0.0, stream=s)
+    torch.cuda.synchronize()
+
+    def work():
+        m.insert(dk, dv, target_lf=0.0, stream=s)
+        m.erase(gone, stream=s)
+
+    g = _captured(s, work)
+    m.clear(stream=s)
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    m.clean_tombstones(stream=s)
+    out = _dev(np.full(n, FILL, _dt(w)))
+    torch.cuda.synchronize()
+    m.retrieve(dk, out, stream=s)
+    want = v.copy()
+    want[: n // 3] = FILL
+    inf = m.info(stream=s)
+    np.testing.assert_array_equal(_host(out, w), want)
+    assert (inf.fill, inf.tombstone_counter, inf.err) == (n - n // 3, 0, hx.STATUS_SUCCESS)
+    m.close()
