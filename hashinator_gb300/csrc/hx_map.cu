@@ -994,13 +994,16 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
 // Growth rule of insert (hashinator.h:1329-1332):
 // ceil(log2((fill + len) / targetLF)) > sizePower -> device_rehash.
 // Decided on the host upper bound of fill; only when that bound asks for
-// growth is the exact fill read back.
+// growth is the exact fill read back. Replays insert past the bound, so it
+// says nothing once an insert was captured (in a capture itself, where nothing
+// can be read back, it is all there is).
 static hx_status maybe_grow(hx_map* m, uint64_t n, float target_lf, cudaStream_t s) {
   if (!(target_lf > 0.0f)) return HX_OK;
   auto needed = [&](uint64_t fill) -> long long {
     return (long long)std::ceil(std::log2((double)(fill + n) * (1.0 / (double)target_lf)));
   };
-  if (needed(m->fill_ub) <= m->sp) return HX_OK;
+  const bool known = !m->replayed || capturing(s);
+  if (known && needed(m->fill_ub) <= m->sp) return HX_OK;
   DInfo di;
   hx_status st = read_info(m, &di, s);
   if (st != HX_OK) return st;

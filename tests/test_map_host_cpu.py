@@ -54,3 +54,18 @@ assert lib.fake_live(0) == held + 1 and lib.fake_live(1) == 0
 m.close()
 assert lib.fake_live(0) == 0
 """)
+
+
+def test_growth_after_a_replay(tmp_path):
+    run_on_host(tmp_path, INFO + """
+def size_power(m):
+    return m.bucket_data()[1].bit_length() - 1
+m = hx.Hashmap(10, 4)
+lib.fake_capture(1)
+m.insert(KEYS, KEYS, n=400, target_lf=0.5)  # in a capture the bound decides: nothing is read back
+lib.fake_capture(0)
+m.clear()
+dinfo().fill = 900  # what a replay leaves
+m.insert(KEYS, KEYS, n=200, target_lf=0.5)
+assert size_power(m) == 12
+""")

@@ -119,3 +119,31 @@ def test_clean_after_a_replay_keeps_every_key(hx, w):
     np.testing.assert_array_equal(_host(out, w), want)
     assert (inf.fill, inf.tombstone_counter, inf.err) == (n - n // 3, 0, hx.STATUS_SUCCESS)
     m.close()
+
+
+@pytest.mark.parametrize("w", [4, 8])
+def test_growth_after_a_replay_counts_its_keys(hx, w):
+    import torch
+    n = 900
+    k, v = workloads.distinct_keys(2 * n, w, 6), workloads.values(2 * n, w, 6)
+    dk, dv = _dev(k), _dev(v)
+    s = torch.cuda.Stream()
+    m = hx.Hashmap(10, w, stream=s)
+    m.insert(dk[:n], dv[:n], target_lf=0.0, stream=s)
+    torch.cuda.synchronize()
+    g = _captured(s, lambda: m.insert(dk[:n], dv[:n], target_lf=0.0, stream=s))
+    m.clear(stream=s)
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    m.insert(dk[n:n + 200], dv[n:n + 200], target_lf=0.5, stream=s)  # 1100 keys
+    inf = m.info(stream=s)
+    assert (inf.fill, inf.err, inf.size_power) == (n + 200, hx.STATUS_SUCCESS, 12)
+    m.insert(dk[n + 200:], dv[n + 200:], target_lf=0.5, stream=s)    # 1800 keys: no growth
+    out = _dev(np.full(2 * n, FILL, _dt(w)))
+    torch.cuda.synchronize()
+    m.retrieve(dk, out, stream=s)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(_host(out, w), v)
+    assert m.info(stream=s).size_power == 12
+    m.close()
