@@ -361,6 +361,7 @@ __global__ void k_batch_clear(P* arena, uint64_t n, DInfo* info, unsigned maps) 
 
 struct hx_batch {
   int key_bytes = 4, val_bytes = 4;
+  int device = 0;
   unsigned n_maps = 0;
   std::vector<int> sp;
   std::vector<unsigned long long> off;
@@ -619,7 +620,7 @@ hx_status hx_batch_create(hx_batch** out, uint32_t n_maps, const int32_t* size_p
     return cuda_status(e);
   };
   cudaError_t e;
-  if ((e = cudaMalloc(&b->arena, acc * pbytes(b))) != cudaSuccess) return fail(e);
+  if ((e = device_alloc(&b->arena, acc * pbytes(b))) != cudaSuccess) return fail(e);
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_off), n_maps * sizeof(unsigned long long))) != cudaSuccess)
     return fail(e);
   if ((e = cudaMalloc(reinterpret_cast<void**>(&b->d_sp), n_maps * sizeof(int))) != cudaSuccess) return fail(e);
@@ -632,7 +633,8 @@ hx_status hx_batch_create(hx_batch** out, uint32_t n_maps, const int32_t* size_p
   *out = b;
   hx_status st = hx_batch_clear(b, stream);
   if (st == HX_OK && (e = cudaStreamSynchronize(s)) != cudaSuccess) st = cuda_status(e);
-  pool_object(+1);
+  cudaGetDevice(&b->device);
+  pool_object(+1, b->device);
   if (st != HX_OK) {
     hx_batch_destroy(b);
     *out = nullptr;
@@ -648,8 +650,8 @@ hx_status hx_batch_destroy(hx_batch* b) {
   cudaFree(b->d_sp);
   cudaFree(b->d_info);
   b->scratch.release();
+  pool_object(-1, b->device);
   delete b;
-  pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);
 }
 
@@ -721,7 +723,7 @@ hx_status hx_batch_plan_create(hx_batch* b, const hx_batch_work* w, hx_batch_pla
       moff[i] = acc;
       acc += cap;
     }
-    cudaError_t e = cudaMalloc(&p->moved, std::max<unsigned long long>(1, acc) * pbytes(b));
+    cudaError_t e = device_alloc(&p->moved, std::max<unsigned long long>(1, acc) * pbytes(b));
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->d_moved_off), nm * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->d_moved_cap), nm * sizeof(unsigned long long));
     if (e == cudaSuccess)

@@ -168,7 +168,7 @@ static hx_status bulk_run(BulkArgs<P> a, BulkSrc src, uint64_t expected, cudaStr
     st = bulk_chunk<P, OP>(a, src, exp1, static_cast<char*>(scratch), s);
   }
   *done = true;
-  HX_CUDA(cudaFreeAsync(scratch, s));
+  HX_CUDA(pool_free(scratch, s));
   return st;
 }
 

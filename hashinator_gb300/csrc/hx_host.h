@@ -61,18 +61,25 @@ int blocks_per_sm(F kernel, int block, size_t smem = 0) {
   return nb;
 }
 
-// Stream-ordered device memory from libhx's own pool of the current device, given
-// back with cudaFreeAsync. The device's default pool hands freed memory to the driver
+// Stream-ordered device memory from libhx's own pool of the current device: scratch of
+// calls and tables that were grown into. The device's default pool hands freed memory to the driver
 // at every synchronisation, so a caller that waits for each result has its scratch
 // mapped anew on every call (the first copy_if of 2^28 words on new arrays: 0.66 ms, with
 // this pool 0.45 ms), and a growing map every new table (2*10^7 u32 keys into a map of the
-// default size, in six chunks: 5.32 ms, with this pool 3.60 ms). This pool keeps up to kPoolKeepBytes of freed memory while a map, batch
-// or server exists, and kPoolIdleBytes once the last one is destroyed (pool_object
-// counts them). Safe with several threads and streams, as any stream-ordered pool is.
-constexpr uint64_t kPoolKeepBytes = 4ull << 30;
+// default size, in six chunks: 5.32 ms, with this pool 3.60 ms). At a synchronisation this
+// pool holds at most kPoolKeepBytes beyond what is in use while a map or batch of the
+// device exists, and kPoolIdleBytes otherwise. The largest scratch of one call is 4.5 GB (2^27
+// u64 pairs slice by slice). Safe with several threads and streams, as any stream-ordered
+// pool is. A server's tables are in a pool of its own.
+constexpr uint64_t kPoolKeepBytes = 5ull << 30;
 constexpr uint64_t kPoolIdleBytes = 1ull << 30;
 cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s);
-void pool_object(int change);  // +1: created, -1: destroyed (after a device synchronisation)
+cudaError_t pool_free(void* p, cudaStream_t s);
+void pool_free_now(void* p);  // after a synchronisation; p may be of cudaMalloc or null
+void pool_trim(uint64_t keep_free);         // of the current device, to what is in use and keep_free
+void pool_object(int change, int dev);      // +1: created, -1: destroyed (after a device synchronisation)
+// cudaMalloc; where the device has no room, once more when the pool has given back what is free.
+cudaError_t device_alloc(void** p, uint64_t bytes);
 
 // Stream-ordered scratch: a caller buffer when given, else pool_alloc
 // on the stream, released stream-ordered by the destructor.

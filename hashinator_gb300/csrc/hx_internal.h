@@ -6,6 +6,7 @@
 #include <vector>
 #include <cuda_runtime.h>
 #include "../../include/hx.h"
+#include "hx_host.h"
 #include "hx_probe.cuh"
 
 namespace hx {
@@ -26,8 +27,8 @@ struct ScratchBuf {
   bool in_graph = false;
   std::vector<void*> kept;
   void release() {  // after a device synchronisation
-    if (ptr) cudaFree(ptr);
-    for (void* p : kept) cudaFree(p);
+    pool_free_now(ptr);
+    for (void* p : kept) pool_free_now(p);
     ptr = nullptr;
     bytes = 0;
     kept.clear();

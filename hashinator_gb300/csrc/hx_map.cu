@@ -874,7 +874,7 @@ class MapScratch {
         return HX_OK;
       }
       if (b.ptr && b.in_graph) b.kept.push_back(b.ptr);
-      else if (b.ptr) HX_CUDA(cudaFreeAsync(b.ptr, stream));
+      else if (b.ptr) HX_CUDA(pool_free(b.ptr, stream));
       b.ptr = nullptr;
       b.bytes = 0;
       b.in_graph = false;
@@ -963,7 +963,7 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
                          held, held}, s, &done);
   if (st != HX_OK) return st;
   if (done) {
-    HX_CUDA(cudaFreeAsync(m->buckets, s));
+    HX_CUDA(pool_free(m->buckets, s));
     m->buckets = nt;
     m->sp = new_sp;
     return HX_OK;
@@ -985,7 +985,7 @@ static hx_status rehash(hx_map* m, int new_sp, cudaStream_t s) {
                                                  new_sp, m->info);
   }
   if ((st = after_launch()) != HX_OK) return st;
-  HX_CUDA(cudaFreeAsync(m->buckets, s));
+  HX_CUDA(pool_free(m->buckets, s));
   m->buckets = nt;
   m->sp = new_sp;
   return HX_OK;
@@ -1129,7 +1129,7 @@ hx_status hx_map_create(hx_map** out, int key_bytes, int val_bytes, int size_pow
     delete m;
     return st;
   };
-  cudaError_t e = cudaMalloc(&m->buckets, nslots(m) * pair_bytes(m));
+  cudaError_t e = device_alloc(&m->buckets, nslots(m) * pair_bytes(m));
   if (e != cudaSuccess) return fail(cuda_status(e));
   e = cudaMalloc(reinterpret_cast<void**>(&m->info), sizeof(DInfo));
   if (e != cudaSuccess) return fail(cuda_status(e));
@@ -1142,18 +1142,18 @@ hx_status hx_map_create(hx_map** out, int key_bytes, int val_bytes, int size_pow
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(cuda_status(e));
   *out = m;
-  pool_object(+1);
+  pool_object(+1, m->device);
   return HX_OK;
 }
 
 hx_status hx_map_destroy(hx_map* m) {
   if (!m) return HX_ERR_INVALID_ARG;
   cudaError_t e = cudaDeviceSynchronize();
-  if (m->buckets) cudaFree(m->buckets);
+  pool_free_now(m->buckets);
   if (m->info) cudaFree(m->info);
   m->own_scratch.release();
+  pool_object(-1, m->device);
   delete m;
-  pool_object(-1);
   return e == cudaSuccess ? HX_OK : cuda_status(e);
 }
 

@@ -3,8 +3,11 @@
 #include <cuda.h>
 
 #include <cstring>
+#include <iterator>
 #include <mutex>
+#include <unordered_map>
 #include "hx_host.h"
+#include "hx_internal.h"
 #include "hx_scan.cuh"
 
 namespace hx {
@@ -66,63 +69,129 @@ unsigned long long current_context_id() {
   return id;
 }
 
-static std::mutex g_pool_mu;
-static struct {
+// libhx's pool of each device, under g_pool_mu.
+struct DevicePool {
   cudaMemPool_t pool;
   unsigned long long ctx;  // the context that it was created in; a reset device has another one
-} g_pools[64];
-static int g_pool_objects = 0;
+  uint64_t in_use;
+  int objects;
+};
+static std::mutex g_pool_mu;
+static DevicePool g_pools[64];
+struct PoolBlock {
+  uint64_t bytes;
+  int dev;
+};
+static std::unordered_map<void*, PoolBlock>& pool_blocks() {
+  static auto* blocks = new std::unordered_map<void*, PoolBlock>();  // never destroyed: handles may outlive main
+  return *blocks;
+}
+
+// The release threshold counts what is in use too, so it follows that.
+static uint64_t pool_keep(const DevicePool& of) {
+  return of.in_use + (of.objects > 0 ? kPoolKeepBytes : kPoolIdleBytes);
+}
+static void pool_set_threshold(const DevicePool& of) {
+  uint64_t keep = pool_keep(of);
+  if (of.pool) cudaMemPoolSetAttribute(of.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+constexpr uint64_t kPoolSmall = kPoolIdleBytes / 64;  // smaller blocks do not move the threshold
 
 cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, s);
+  // a capture takes nothing but stream work, and its memory belongs to the graph
+  if (dev < 0 || dev >= 64 || capturing(s)) return cudaMallocAsync(p, bytes, s);
   std::lock_guard<std::mutex> g(g_pool_mu);
   const unsigned long long ctx = current_context_id();
-  auto& of = g_pools[dev];
+  DevicePool& of = g_pools[dev];
   if (ctx && (!of.pool || of.ctx != ctx)) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      return cudaMallocAsync(p, bytes, s);  // nothing but stream work while a capture runs
-    }
+    auto& blocks = pool_blocks();
+    for (auto it = blocks.begin(); it != blocks.end();) it = it->second.dev == dev ? blocks.erase(it) : std::next(it);
+    of.pool = nullptr;
+    of.in_use = 0;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    of.pool = nullptr;
     cudaMemPool_t made = nullptr;
     if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
-      uint64_t keep = kPoolKeepBytes;
-      cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
       of.pool = made;
       of.ctx = ctx;
+      pool_set_threshold(of);
     } else {
       cudaGetLastError();
     }
   }
   if (!ctx || !of.pool) return cudaMallocAsync(p, bytes, s);
   e = cudaMallocFromPoolAsync(p, bytes, of.pool, s);
-  if (e == cudaSuccess && bytes >= kPoolKeepBytes / 256) {
-    // the threshold counts what is in use too (grown tables): keep kPoolKeepBytes beyond that
-    uint64_t used = 0;
-    if (cudaMemPoolGetAttribute(of.pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
-      used += kPoolKeepBytes;
-      cudaMemPoolSetAttribute(of.pool, cudaMemPoolAttrReleaseThreshold, &used);
-    }
+  if (e == cudaErrorMemoryAllocation) {  // freed blocks of other sizes may be in the way
+    cudaGetLastError();
+    cudaMemPoolTrimTo(of.pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, of.pool, s);
   }
-  return e;
+  if (e != cudaSuccess) return e;
+  pool_blocks()[*p] = PoolBlock{bytes, dev};
+  of.in_use += bytes;
+  if (bytes >= kPoolSmall) pool_set_threshold(of);
+  return cudaSuccess;
 }
 
-void pool_object(int change) {
+// Takes p off the books if it is a block of the pool.
+static void pool_forget(void* p) {
   std::lock_guard<std::mutex> g(g_pool_mu);
-  g_pool_objects += change;
-  if (change > 0 || g_pool_objects > 0) return;
+  auto& blocks = pool_blocks();
+  const auto it = blocks.find(p);
+  if (it == blocks.end()) return;
+  DevicePool& of = g_pools[it->second.dev];
+  const uint64_t bytes = it->second.bytes;
+  of.in_use -= bytes;
+  blocks.erase(it);
+  if (bytes >= kPoolSmall) pool_set_threshold(of);
+}
+cudaError_t pool_free(void* p, cudaStream_t s) {
+  pool_forget(p);
+  return cudaFreeAsync(p, s);
+}
+void pool_free_now(void* p) {
+  if (!p) return;
+  pool_forget(p);
+  cudaFree(p);
+}
+
+void pool_trim(uint64_t keep_free) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-  const auto& of = g_pools[dev];
-  if (of.pool && of.ctx == current_context_id()) cudaMemPoolTrimTo(of.pool, kPoolIdleBytes);
+  std::lock_guard<std::mutex> g(g_pool_mu);
+  const DevicePool& of = g_pools[dev];
+  if (of.pool && of.ctx == current_context_id()) cudaMemPoolTrimTo(of.pool, of.in_use + keep_free);
+}
+
+void pool_object(int change, int dev) {
+  if (dev < 0 || dev >= 64) return;
+  int current = dev;
+  cudaGetDevice(&current);
+  if (current != dev && cudaSetDevice(dev) != cudaSuccess) return;
+  {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    DevicePool& of = g_pools[dev];
+    of.objects += change;
+    if (of.pool && of.ctx == current_context_id()) {
+      pool_set_threshold(of);
+      if (change < 0) cudaMemPoolTrimTo(of.pool, pool_keep(of));
+    }
+  }
+  if (current != dev) cudaSetDevice(current);
+}
+
+cudaError_t device_alloc(void** p, uint64_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  cudaDeviceSynchronize();  // what was freed on a stream is free then
+  pool_trim(0);
+  return cudaMalloc(p, bytes);
 }
 
 hx_status Scratch::get(void* caller, uint64_t caller_bytes, uint64_t need, cudaStream_t stream) {
@@ -139,7 +208,7 @@ hx_status Scratch::get(void* caller, uint64_t caller_bytes, uint64_t need, cudaS
 }
 
 Scratch::~Scratch() {
-  if (owned && ptr) cudaFreeAsync(ptr, s);
+  if (owned && ptr) pool_free(ptr, s);
 }
 
 // Reads the count and error word back for a synchronous call.

@@ -357,6 +357,16 @@ namespace hx {
 
 static uint64_t pb(const hx_server* sv) { return sv->kb == 4 ? 8 : 16; }
 
+// A table from the server's pool; where the device has no room, once more when libhx's
+// own pool has given back what is free.
+static cudaError_t table_alloc(hx_server* sv, void** p, uint64_t bytes) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, sv->pool, sv->s);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  pool_trim(0);
+  return cudaMallocFromPoolAsync(p, bytes, sv->pool, sv->s);
+}
+
 static void view_of(hx_server* sv, unsigned i, hx_map* v) {
   v->key_bytes = sv->kb;
   v->val_bytes = sv->kb;
@@ -572,7 +582,7 @@ hx_status hx_server_add_map(hx_server* sv, int size_power, uint32_t* map_id) {
   ServeMap m;
   m.sp = size_power;
   m.bytes = bytes;
-  HX_CUDA(cudaMallocFromPoolAsync(&m.table, bytes, sv->pool, sv->s));
+  HX_CUDA(table_alloc(sv, &m.table, bytes));
   hx_map v;
   v.key_bytes = sv->kb;
   v.val_bytes = sv->kb;
@@ -668,7 +678,7 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
     const uint64_t nbytes = (1ull << nsp) * pb(sv);
     int& slot_of = grow_of[map];
     void* nt = nullptr;
-    const cudaError_t e = cudaMallocFromPoolAsync(&nt, nbytes, sv->pool, sv->s);
+    const cudaError_t e = table_alloc(sv, &nt, nbytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return e;

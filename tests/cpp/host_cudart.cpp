@@ -28,7 +28,10 @@ int g_fail_host = 0;       // the next so many page-locked allocations fail
 bool g_capturing = false;
 cudaError_t g_last = cudaSuccess;
 
+uint64_t g_capacity = ~0ull;  // bytes of the device
+
 cudaError_t fail(cudaError_t e) { return g_last = e; }
+uint64_t taken();  // by the pools, and by allocations outside them
 cudaError_t make(void** p, size_t bytes, bool host = false) {
   const size_t page = 4096, body = (bytes + page - 1) / page * page + (bytes ? 0 : page);
   char* m = static_cast<char*>(mmap(nullptr, body + page, PROT_READ | PROT_WRITE,
@@ -61,6 +64,12 @@ struct Pools {
         p.first->held = p.first->used > p.first->threshold ? p.first->used : p.first->threshold;
   }
 } g_pools;
+uint64_t taken() {
+  uint64_t n = 0;
+  for (auto& p : g_pools.all) n += p.first->held;
+  for (auto& b : g_live) n += b.second.host || g_of_pool.count(b.first) ? 0 : b.second.bytes;
+  return n;
+}
 dim3 g_grid, g_block;
 size_t g_smem;
 cudaStream_t g_stream;
@@ -78,6 +87,7 @@ int fake_live(int captured) {  // live device allocations: made under capture, o
   return n;
 }
 void fake_fail_pool_from(size_t bytes) { g_fail_from = bytes; }
+void fake_capacity(uint64_t bytes) { g_capacity = bytes; }
 void fake_fail_host(int count) { g_fail_host = count; }
 void fake_capture(int on) { g_capturing = on != 0; }
 uint64_t fake_pool_held() {  // bytes that every pool holds once all work is done
@@ -110,7 +120,10 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) 
 cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return cudaSuccess; }
 
-cudaError_t cudaMalloc(void** p, size_t n) { return make(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) {
+  if (g_capacity != ~0ull && taken() + n > g_capacity) return fail(cudaErrorMemoryAllocation);
+  return make(p, n);
+}
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return make(p, n); }
 cudaError_t cudaMallocHost(void** p, size_t n) {
   if (g_fail_host > 0) {
@@ -134,9 +147,11 @@ cudaError_t cudaMemPoolDestroy(cudaMemPool_t p) {
 }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t pool, cudaStream_t) {
   if (g_fail_from && n >= g_fail_from) return fail(cudaErrorMemoryAllocation);
+  Pool* q = reinterpret_cast<Pool*>(pool);
+  if (g_capacity != ~0ull && q->used + n > q->held && taken() + (q->used + n - q->held) > g_capacity)
+    return fail(cudaErrorMemoryAllocation);
   const cudaError_t e = make(p, n);
   if (e != cudaSuccess) return e;
-  Pool* q = reinterpret_cast<Pool*>(pool);
   g_of_pool[*p] = q;
   q->used += n;
   if (q->held < q->used) q->held = q->used;

@@ -19,6 +19,7 @@ lib.fake_find.restype = ctypes.c_void_p
 lib.fake_find.argtypes = [ctypes.c_size_t]
 lib.fake_fail_pool_from.argtypes = [ctypes.c_size_t]
 lib.fake_pool_held.restype = ctypes.c_uint64
+lib.fake_capacity.argtypes = [ctypes.c_uint64]
 KEYS = 1 << 20  # an address: nothing reads it here
 """
 
