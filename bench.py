@@ -11,10 +11,12 @@ value: device-resident inputs, CUDA events around the K timed steps.
 e2e:   the same step through the C ABI with pinned HOST buffers: the H2D copy
        of keys, values and queries and the D2H copy of the query results are
        inside the timed region.
-roofline: the dominant kernel's algorithmic bytes (insert 72 B/key, query
-       40 B/key: key+value in, one 32 B bucket sector read, written back for
-       insert) over its event-timed duration, against the measured HBM copy
-       bandwidth (MEASURED_PEAKS.json).
+roofline: the algorithmic bytes of the slower of insert and query over its
+       event-timed duration, against the measured HBM copy bandwidth
+       (MEASURED_PEAKS.json). A batch that goes slice by slice through the table
+       moves its keys and values once and the table once (once more back for
+       insert); one that probes directly moves key, value and one 32 B bucket
+       sector a key, written back for insert (insert 72 B/key, query 40 B/key).
 cpu_baseline: the oracle's serial C restatement of the reference's CPU path on
        a bounded sample (2^24 keys into 2^25 buckets, same load factor), as
        one serial map per host thread (keys sharded by home bucket) and on one
@@ -43,7 +45,7 @@ import numpy as np
 ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
-INSERT_BYTES_PER_KEY = {4: 72, 8: 80}
+INSERT_BYTES_PER_KEY = {4: 72, 8: 80}  # probing directly
 QUERY_BYTES_PER_KEY = {4: 40, 8: 48}
 HEADLINE_FILL = 0xA5A5A5A5  # query-output pre-fill of the headline step
 METRIC = "insert+query Mkeys/s (u32 keys/values, 2^26 keys, 2^27 buckets, LF 0.5, 50% hit queries)"
@@ -75,7 +77,7 @@ def measured_peak():
 
 
 def traffic_from_profiles(kernel_tag: str):
-    """Per-launch DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one kernel at the headline size,
+    """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one insert or query call at the headline size,
     from the ncu capture recorded in profiles/roofline_traffic.json (each entry carries the command that
     produced it), or None when no capture of that kernel exists."""
     p = ROOT / "profiles" / "roofline_traffic.json"
@@ -936,21 +938,25 @@ def run_ours(args):
     if args.group:
         m.set_tuning(group_width=args.group)
 
-    def step(ev=None):
-        if ev:
-            ev[0].record(stream)
+    def step(ev=None, kernels=None):
+        def mark(i):
+            if ev:
+                ev[i].record(stream)
+            if kernels is not None:
+                kernels.append(hx.kernel_launch_count())
+
+        mark(0)
         m.clear(stream=stream)
-        if ev:
-            ev[1].record(stream)
+        mark(1)
         m.insert(d_keys, d_vals, target_lf=0.5, stream=stream)
-        if ev:
-            ev[2].record(stream)
+        mark(2)
         m.retrieve(d_q, d_out, stream=stream)
-        if ev:
-            ev[3].record(stream)
+        mark(3)
 
     for _ in range(args.warmup):
-        step()
+        at = []
+        step(kernels=at)
+    kernels_of = {"insert": at[2] - at[1], "query": at[3] - at[2]}  # more than one: slice by slice through the table
     torch.cuda.synchronize()
     # every retrieve output of the warm-up steps, element for element (not timed)
     host_out = d_out.cpu().numpy().view(np.uint32)
@@ -1166,28 +1172,45 @@ def run_ours(args):
     del rbuf
 
     peak, peak_kind = measured_peak()
-    ins_gbs = INSERT_BYTES_PER_KEY[width] * n / t_ins / 1e9
-    q_gbs = QUERY_BYTES_PER_KEY[width] * n / t_q / 1e9
     dominant = "insert" if t_ins >= t_q else "query"
+    by_slices = kernels_of[dominant] > 1
+
+    def call_bytes(op):
+        if kernels_of[op] > 1:
+            return 2 * width * n + (2 * width << sp) * (2 if op == "insert" else 1)
+        return (INSERT_BYTES_PER_KEY if op == "insert" else QUERY_BYTES_PER_KEY)[width] * n
+
+    ins_gbs = call_bytes("insert") / t_ins / 1e9
+    q_gbs = call_bytes("query") / t_q / 1e9
     achieved = ins_gbs if dominant == "insert" else q_gbs
-    # measured traffic (2^26 keys) exists for the thread-per-key insert and query kernels
-    tag = ("insert_u32_lf050" if args.group in (0, 1) else None) if dominant == "insert" else \
-        ("query_t1_u32_lf050" if args.group == 1 else ("query_u32_lf050" if args.group == 0 else None))
+    # measured traffic (2^26 keys) exists for the default calls, the thread-per-key kernels and 4-lane queries
+    tag = {("insert", 1): "insert_t1_u32_lf050", ("query", 1): "query_t1_u32_lf050",
+           ("query", 4): "query_u32_lf050"}.get((dominant, args.group))
+    if args.group == 0 and by_slices:
+        tag = f"{dominant}_slices_u32_lf050"
     traffic = traffic_from_profiles(tag) if tag and args.log_keys == 26 else None
     dom_keys_s = n / (t_ins if dominant == "insert" else t_q)
+    if by_slices:
+        kernel = "k_bulk_split, k_bulk_slice, " + ("k_bulk_left (insert)" if dominant == "insert" else
+                                                   "k_bulk_scatter, k_bulk_left (query)")
+        random_frac = None
+        random_note = ("ceilings measured in this run by hx_diag_random_access over 1 GiB; they bound batches that "
+                       "probe directly, not one that goes slice by slice through the table")
+    else:
+        kernel = {("insert", 0): "k_insert_queue", ("insert", 1): "k_insert_t1", ("query", 0): "k_find_queue",
+                  ("query", 1): "k_find_t1"}.get((dominant, args.group),
+                                                 "k_insert" if dominant == "insert" else "k_retrieve") + f" ({dominant})"
+        random_frac = round(dom_keys_s / (ceil[1] if dominant == "insert" else ceil[0]), 3)
+        random_note = ("ceilings measured in this run by hx_diag_random_access over 1 GiB; frac = keys/s of the "
+                       "dominant kernel over the ceiling of its one unavoidable random op per key (CAS for "
+                       "insert, 32-byte read for query); DRAM transactions, not bytes, bound these kernels")
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": f"{peak_kind} hbm_gbs",
                 "random_access": {
                     "read32_G_per_s": round(ceil[0] / 1e9, 2), "cas64_G_per_s": round(ceil[1] / 1e9, 2),
-                    "frac": round(dom_keys_s / (ceil[1] if dominant == "insert" else ceil[0]), 3),
-                    "note": "ceilings measured in this run by hx_diag_random_access over 1 GiB; frac = keys/s of the "
-                            "dominant kernel over the ceiling of its one unavoidable random op per key (CAS for "
-                            "insert, 32-byte read for query); DRAM transactions, not bytes, bound these kernels"},
-                "kernel": (("k_insert_t1 (insert)" if args.group in (0, 1) else "k_insert (insert)")
-                           if dominant == "insert" else
-                           ("k_find_t1 (query)" if args.group == 1 else "k_retrieve (query)")),
-                "algorithmic_bytes_per_launch": (INSERT_BYTES_PER_KEY if dominant == "insert"
-                                                 else QUERY_BYTES_PER_KEY)[width] * n,
+                    "frac": random_frac, "note": random_note},
+                "kernel": kernel, "kernels_per_call": kernels_of[dominant],
+                "algorithmic_bytes_per_launch": call_bytes(dominant),
                 "per_op": {"insert": {"ms": round(t_ins * 1e3, 3), "Mkeys_s": round(n / t_ins / 1e6, 1),
                                       "GB_s": round(ins_gbs, 1), "frac": round(ins_gbs / peak, 4)},
                            "query": {"ms": round(t_q * 1e3, 3), "Mkeys_s": round(n / t_q / 1e6, 1),
