@@ -188,6 +188,14 @@ static hx_status bulk_run(BulkArgs<P> a, BulkSrc src, uint64_t expected, cudaStr
 //                     1/15 1.34 / 1.62; look-up [128] 1/5 1.0 / 1.34, [256] 1/5 1.45 / 2.4
 //   load factor 0.92: insert [32] 1/4 2.0 / 4.1; erase [32] 1/14 2.8 / 5.4; look-up
 //                     [32] 1/4 2.1 / 2.2, [128] 2.2 / 3.3
+// What the host cannot tell, direct time over slice time. Look-ups of keys all absent /
+// half / all present, load factor 0.5: u32 [512 MiB] 1.48 / 1.08 / 0.99, [1 GiB] 1.81 /
+// 1.29 / 1.12; u64 [2 GiB] 1.78 / 1.09 / 0.86, [4 GiB] 1.81 / 1.11 / 0.88. Batches that do
+// not spread over the table (2^26 u32 keys, 2^27 buckets): every second key the same,
+// insert 4.5, look-up 0.73, erase 1.7; zipf(1) 5.8 / 0.79 / 1.7; 1024 distinct keys 2.5 /
+// 0.71 / 2.1; keys in bucket order 0.54 / 0.99 / 0.44. A rehash of 2^27 u64 buckets 1.14
+// with keys spread over 64 bits, 0.86 with keys below 2^(64 - sp), whose old and new
+// buckets are in one order.
 // The load factor is the host's bound of it (after the inserts of this call); a bound
 // above the table's size says nothing, and counts as a low one.
 static unsigned bulk_spread(BulkOp op, bool p32, uint64_t bytes, double lf) {

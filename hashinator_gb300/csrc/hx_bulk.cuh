@@ -10,7 +10,10 @@
 //      the top bits of their home bucket. A tile is binned in shared memory
 //      and leaves as one contiguous run per bin.
 //   2. slice: one CTA per slice of 32 KiB of buckets reads it, looks the bin's
-//      keys up in shared memory, and writes the buckets that change.
+//      keys up in shared memory, and writes the buckets that change, and only
+//      those: the CTA of the slice before may at the same time write values and
+//      TOMBSTONEs into this slice's first buckets (its own keys that sit past its
+//      end), which a write of the whole slice would undo.
 //   3. left: a key that may belong past the end of its slice is handled in the
 //      whole table, after every slice.
 //   4. scatter (look-ups): the values found leave step 2 binned by their place

@@ -1,12 +1,14 @@
 // hx_map.cu — Hashinator::Hashmap accelerated API on device-resident tables.
 //
 // Kernels: insert (keys+values or pairs), retrieve (keys or pairs), erase,
-// device rehash, clear, and the clean_tombstones pair (compaction in clean
-// mode + re-insert). All hash kernels are persistent grid-stride kernels:
-// a warp takes 32/G consecutive keys per step (one per probe group), so key
-// loads are coalesced; fill / tombstone / probe-bound updates are reduced per
-// warp and applied with one atomic per warp at kernel exit (the reference
-// reduces per block, kernels_NVIDIA.h:411-440).
+// device rehash and clear; clean_tombstones is k_clean (hx_clean.cuh), and large
+// batches go slice by slice through the table (hx_bulk.cu). The hash kernels here
+// probe the table directly and are persistent grid-stride kernels: one key per
+// thread, with the probes that go on in a queue of their warp, or one per group of G
+// lanes (a warp then takes 32/G consecutive keys per step), so key loads are
+// coalesced; fill / tombstone / probe-bound updates are reduced per warp and applied
+// with one atomic per warp at kernel exit (the reference reduces per block,
+// kernels_NVIDIA.h:411-440).
 #include <cmath>
 #include <cstring>
 #include <mutex>

@@ -155,7 +155,8 @@ hx_status hx_erase(hx_map* map, const void* d_keys, uint64_t n, hx_stream stream
 /* clean_tombstones(stream) (hashinator.h:1262-1315): every TOMBSTONE bucket
  * becomes EMPTY and every key that does not sit in its home bucket is taken
  * out and inserted again; fill is unchanged, tombstone_counter becomes 0.
- * Uses a map-owned device buffer (grown on demand) for the moved keys. */
+ * Uses a map-owned device buffer (grown on demand) for the keys that leave
+ * their slice of the table. */
 hx_status hx_clean_tombstones(hx_map* map, hx_stream stream);
 
 /* extractPattern(hash_pair*, Rule, stream) (hashinator.h:1168-1185) and

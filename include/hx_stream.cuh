@@ -31,7 +31,10 @@
 // at 42%. Two groups fill each other's waits, and the write-out of one phase no
 // longer waits for pass 1 of the next. 2^28 u32, 1 / 25 / 50 / 75 / 99 of 100
 // selected: 304 / 340 / 373 / 419 / 473 us with every thread in both passes,
-// 280 / 305 / 332 / 366 / 420 so. Pairs out of 2^27 buckets: 371 -> 331 us.
+// 280 / 305 / 332 / 366 / 420 so. Pairs out of 2^27 buckets: 371 -> 331 us. A caller's
+// rule that computes much gains nothing and can lose: 2^27 u32 by 32 hash rounds 1.15 ->
+// 1.22 ms, by sinf, expf, logf and cosf 0.90 -> 1.13 ms; fewer writers, for more registers
+// a thread, do not help it (1.10 - 1.17 ms with 128 - 256).
 //
 // Co-residency: every CTA waits for the counts of every other, so the launch
 // is cooperative (the runtime guarantees all CTAs resident). Every wait is
