@@ -14,13 +14,16 @@ def _free():
 
 
 def test_freed_tables_go_back_to_the_device(hx):
+    import gc
     import torch
+    gc.collect()  # maps of earlier tests
     torch.cuda.empty_cache()
+    hx.Hashmap(10, 4).close()
+    start = _free()  # the pool may still hold the 1 GiB that it keeps without a map
     small = hx.Hashmap(10, 4)
-    start = _free()
     big = hx.Hashmap(20, 8)
     big.resize(30)  # 16 GiB
-    assert start - _free() >= 16 * GIB
+    assert start - _free() >= 15 * GIB
     big.resize(22)
     assert start - _free() <= 5 * GIB + (1 << 27)
     big.resize(30)
