@@ -860,14 +860,22 @@ static hx_status launch_find(hx_map* m, const void* keys, void* vals, void* pair
   return after_launch();
 }
 
+// A call under capture runs again with every replay of its graph, which the host does
+// not see: from then on it takes nothing for known that such a replay may change.
+// Whether this call is one.
+static bool note_capture(hx_map* m, cudaStream_t s) {
+  const bool captured = capturing(s);
+  m->replayed |= captured;
+  return captured;
+}
+
 // The map's scratch for one call. In a capture, where the map's buffer cannot be
 // replaced, a larger need is met by memory of the graph's own.
 class MapScratch {
  public:
   void* ptr = nullptr;
-  hx_status get(hx_map* m, uint64_t bytes, cudaStream_t stream) {
+  hx_status get(hx_map* m, uint64_t bytes, cudaStream_t stream, bool captured) {
     ScratchBuf& b = *m->scratch;
-    const bool captured = capturing(stream);
     if (b.bytes < bytes) {
       if (captured) {
         HX_CUDA(cudaMallocAsync(&ptr, bytes, stream));
@@ -910,12 +918,13 @@ static hx_status launch_clean(hx_map* m, cudaStream_t s) {
   MapScratch list;
   hx_status st;
   if (grid > 1) {
+    const bool captured = note_capture(m, s);
+    m->err_success = false;  // the kernels may set fail
     // Listed keys <= fill, and fill <= fill_ub unless replays or a caller's kernels insert
     // unseen: then there is room for every bucket.
     cap = m->fill_ub < n && !m->replayed && !m->viewed ? m->fill_ub : n;
-    if ((st = list.get(m, cap * sizeof(P), s)) != HX_OK) return st;
+    if ((st = list.get(m, cap * sizeof(P), s, captured)) != HX_OK) return st;
   }
-  m->err_success = false;  // the kernels may set fail
   constexpr int PER = 32 / sizeof(P);
   auto launch = [&](auto kern) -> hx_status {
     const size_t smem = clean_smem<P>(slots);
@@ -1025,12 +1034,6 @@ static hx_status try_bulk(const hx_map* m, BulkOp op, const void* keys, const vo
                   s, done);
 }
 
-// A call under capture runs again with every replay of its graph, which the host does
-// not see: from then on it takes nothing for known that such a replay may change.
-static void note_capture(hx_map* m, cudaStream_t s) {
-  if (!m->replayed && capturing(s)) m->replayed = true;
-}
-
 // err = success before an insert (hashers.h:50), unless the device word is known to
 // hold it: after a clear, until a kernel that may set fail, a peek_status, a device
 // view (whose kernels write it unseen) or a captured call (whose replays do).
@@ -1080,7 +1083,7 @@ static hx_status extract(hx_map* m, const hx_pred* pred, void* d_out, uint64_t c
   const uint64_t need = p32 ? compact_scratch_need<P32>(n) : compact_scratch_need<P64>(n);
   const uint64_t sc_bytes = (need + 255) / 256 * 256;
   MapScratch sc;
-  hx_status st = sc.get(m, sc_bytes + 256, s);
+  hx_status st = sc.get(m, sc_bytes + 256, s, capturing(s));
   if (st != HX_OK) return st;
   unsigned long long* cnt = d_count ? reinterpret_cast<unsigned long long*>(d_count)
                                     : reinterpret_cast<unsigned long long*>(static_cast<char*>(sc.ptr) + sc_bytes);
@@ -1258,7 +1261,6 @@ hx_status hx_clean_tombstones(hx_map* m, hx_stream stream) {
   if (!valid_map(m)) return HX_ERR_INVALID_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::lock_guard<std::mutex> g(m->mu);
-  note_capture(m, s);
   return is_p32(m) ? launch_clean<P32>(m, s) : launch_clean<P64>(m, s);
 }
 
