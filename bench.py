@@ -605,7 +605,8 @@ def run_lf_sweep(args, stream, dev, peak):
             return torch.from_numpy(np.ascontiguousarray(a).view(sig)).to(dev)
 
         dk, dv = dev_t(keys), dev_t(vals)
-        ib, qb, eb = {4: 72, 8: 80}[width], {4: 40, 8: 48}[width], {4: 68, 8: 72}[width]
+        eb = {4: 68, 8: 72}[width]  # an erase that probes directly
+        pb, table = 2 * width, 2 * width << sp
         for lf in (0.5, 0.75, 0.9):
             n = int(lf * (1 << sp))
             rng = np.random.default_rng(int(lf * 100) + width)
@@ -630,17 +631,26 @@ def run_lf_sweep(args, stream, dev, peak):
             t_clear = _ev_time(stream, lambda: m.clear(stream=stream))
             t_ins -= t_clear
             m.clear(stream=stream)
+            l0 = hx.kernel_launch_count()  # more than one kernel a call: slice by slice through the table
             m.insert(dk[:n], dv[:n], target_lf=0.0, stream=stream)
+            l1 = hx.kernel_launch_count()
+            m.retrieve(dq, o, stream=stream)
+            l2 = hx.kernel_launch_count()
+            ins_bytes = pb * n + 2 * table if l1 - l0 > 1 else INSERT_BYTES_PER_KEY[width] * n
+            q_bytes = pb * n + table if l2 - l1 > 1 else QUERY_BYTES_PER_KEY[width] * n
             t_q = _ev_time(stream, lambda: m.retrieve(dq, o, stream=stream))
             # a clean with no tombstones skips its pass but sizes the map's scratch, so the timed clean
             # below measures the pass, not a first-time stream-ordered allocation
             m.clean_tombstones(stream=stream)
             exact = bool(np.array_equal(o.cpu().numpy().view(keys.dtype), expect))
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            l0 = hx.kernel_launch_count()
             e0.record(stream)
             m.erase(de, stream=stream)
             e1.record(stream)
             torch.cuda.synchronize()
+            e_bytes = (width * len(ee) + table + min(pb * len(ee), table) if hx.kernel_launch_count() - l0 > 1
+                       else eb * len(ee))
             t_e = e0.elapsed_time(e1) / 1e3
             e0.record(stream)
             m.clean_tombstones(stream=stream)
@@ -654,14 +664,13 @@ def run_lf_sweep(args, stream, dev, peak):
             expect2 = expect.copy()
             expect2[erased_q] = fill
             exact2 = bool(np.array_equal(o.cpu().numpy().view(keys.dtype), expect2))
-            pb = 8 if width == 4 else 16
             moved = int(inf.last_clean_moved)
-            clean_bytes = (1 << sp) * pb + ib * moved  # scan of every bucket + one insert per moved key
+            clean_bytes = 2 * table  # every bucket read and written once
             out.append({"key_bytes": width, "load_factor": lf, "keys": n,
-                        "insert_Mkeys_s": round(n / t_ins / 1e6, 1), "insert_frac": round(n * ib / t_ins / 1e9 / peak, 4),
-                        "query_Mkeys_s": round(n / t_q / 1e6, 1), "query_frac": round(n * qb / t_q / 1e9 / peak, 4),
+                        "insert_Mkeys_s": round(n / t_ins / 1e6, 1), "insert_frac": round(ins_bytes / t_ins / 1e9 / peak, 4),
+                        "query_Mkeys_s": round(n / t_q / 1e6, 1), "query_frac": round(q_bytes / t_q / 1e9 / peak, 4),
                         "erase_Mkeys_s": round(len(ee) / t_e / 1e6, 1),
-                        "erase_frac": round(len(ee) * eb / t_e / 1e9 / peak, 4),
+                        "erase_frac": round(e_bytes / t_e / 1e9 / peak, 4),
                         "clean_ms": round(t_c * 1e3, 3), "clean_moved": moved,
                         "clean_GB_s": round(clean_bytes / t_c / 1e9, 1),
                         "clean_frac": round(clean_bytes / t_c / 1e9 / peak, 4),
@@ -672,9 +681,10 @@ def run_lf_sweep(args, stream, dev, peak):
             del dq, de, o
         del dk, dv
         torch.cuda.empty_cache()
-    return {"note": "fraction of the measured HBM copy bandwidth for algorithmic bytes (insert 72/80, query 40/48, "
-                    "erase 68/72 B per key; clean_tombstones 8/16 B per bucket scanned + 72/80 B per moved key); "
-                    "query_exact/requery_exact compare every query output with the known answer",
+    return {"note": "fraction of the measured HBM copy bandwidth for algorithmic bytes (slice by slice: keys and values "
+                    "once and the table once, written back for insert, the erased keys' buckets for erase; probing "
+                    "directly: insert 72/80, query 40/48, erase 68/72 B per key; clean_tombstones: every bucket read "
+                    "and written); query_exact/requery_exact compare every query output with the known answer",
             "runs": out}
 
 

@@ -68,8 +68,8 @@ int blocks_per_sm(F kernel, int block, size_t smem = 0) {
 // this pool 0.45 ms), and a growing map every new table (2*10^7 u32 keys into a map of the
 // default size, in six chunks: 5.32 ms, with this pool 3.60 ms). At a synchronisation this
 // pool holds at most kPoolKeepBytes beyond what is in use while a map or batch of the
-// device exists, and kPoolIdleBytes otherwise. The largest scratch of one call is 4.5 GB (2^27
-// u64 pairs slice by slice). Safe with several threads and streams, as any stream-ordered
+// device exists, and kPoolIdleBytes otherwise. Scratch of one call: 4.6 GB at most for
+// look-ups; for inserts 6.4 GB (2^27 u64 pairs into 2^29 buckets), 4.8 GB into 2^27. Safe with several threads and streams, as any stream-ordered
 // pool is. A server's tables are in a pool of its own.
 constexpr uint64_t kPoolKeepBytes = 5ull << 30;
 constexpr uint64_t kPoolIdleBytes = 1ull << 30;

@@ -14,6 +14,21 @@
  * (hashinator/hashers.h:55,76,98,118,128,140,151,161); a caller that wants
  * that behaviour calls cudaStreamSynchronize, or hx_get_info, afterwards.
  *
+ * Device memory: hx_insert*, hx_retrieve* and hx_erase of large batches on
+ * large tables, and hx_resize, take stream-ordered scratch for the length of
+ * the call (two records a key, 9 - 48 bytes together, at most 6.5 GB); if
+ * it cannot be had they run without it. Scratch, and tables that were grown
+ * into, come from a memory pool of the library's own, which at a
+ * synchronisation holds at most 5 GiB beyond what is in use while a map or
+ * batch of the device exists, and 1 GiB otherwise. Its free memory is given
+ * back when an allocation of the library finds no room; other libraries in
+ * the process see it as taken.
+ *
+ * Stream capture: a captured call takes no scratch of that pool, and large
+ * batches then probe the table directly. A graph that holds an insert, clean
+ * or resize of a map may be replayed between other calls on it: they then
+ * take nothing from what the host knew of the map's contents.
+ *
  * Each declaration names the reference interface it replaces
  * (path:line inside the Hashinator source tree, version 1.0.1).
  */
