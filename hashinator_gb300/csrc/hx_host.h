@@ -73,7 +73,9 @@ int blocks_per_sm(F kernel, int block, size_t smem = 0) {
 // pool is. A server's tables are in a pool of its own.
 constexpr uint64_t kPoolKeepBytes = 5ull << 30;
 constexpr uint64_t kPoolIdleBytes = 1ull << 30;
-cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s);
+// counted: in the count of what is in use, and given back with pool_free; not counted: a
+// small buffer of one call, given back with cudaFreeAsync.
+cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s, bool counted = true);
 cudaError_t pool_free(void* p, cudaStream_t s);
 void pool_free_now(void* p);  // after a synchronisation; p may be of cudaMalloc or null
 void pool_trim(uint64_t keep_free);         // of the current device, to what is in use and keep_free

@@ -97,16 +97,17 @@ static void pool_set_threshold(const DevicePool& of) {
 }
 constexpr uint64_t kPoolSmall = kPoolIdleBytes / 64;  // smaller blocks do not move the threshold
 
-cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s) {
+cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s, bool counted) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  // a capture takes nothing but stream work, and its memory belongs to the graph
-  if (dev < 0 || dev >= 64 || capturing(s)) return cudaMallocAsync(p, bytes, s);
+  // memory of a capture belongs to its graph
+  if (dev < 0 || dev >= 64 || (counted && capturing(s))) return cudaMallocAsync(p, bytes, s);
   std::lock_guard<std::mutex> g(g_pool_mu);
   const unsigned long long ctx = current_context_id();
   DevicePool& of = g_pools[dev];
   if (ctx && (!of.pool || of.ctx != ctx)) {
+    if (capturing(s)) return cudaMallocAsync(p, bytes, s);  // nothing but stream work while a capture runs
     auto& blocks = pool_blocks();
     for (auto it = blocks.begin(); it != blocks.end();) it = it->second.dev == dev ? blocks.erase(it) : std::next(it);
     of.pool = nullptr;
@@ -131,7 +132,7 @@ cudaError_t pool_alloc(void** p, uint64_t bytes, cudaStream_t s) {
     cudaMemPoolTrimTo(of.pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, of.pool, s);
   }
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !counted) return e;
   pool_blocks()[*p] = PoolBlock{bytes, dev};
   of.in_use += bytes;
   if (bytes >= kPoolSmall) pool_set_threshold(of);
@@ -202,13 +203,13 @@ hx_status Scratch::get(void* caller, uint64_t caller_bytes, uint64_t need, cudaS
     owned = false;
     return HX_OK;
   }
-  HX_CUDA(pool_alloc(&ptr, need, stream));
+  HX_CUDA(pool_alloc(&ptr, need, stream, false));
   owned = true;
   return HX_OK;
 }
 
 Scratch::~Scratch() {
-  if (owned && ptr) pool_free(ptr, s);
+  if (owned && ptr) cudaFreeAsync(ptr, s);
 }
 
 // Reads the count and error word back for a synchronous call.

@@ -403,9 +403,8 @@ static uint64_t round_tile(uint64_t round_keys) { return round_keys < (1ull << 2
 // Room for the tiles of a round. A request above the round's limit of keys runs alone,
 // however large it is, so a slot's buffers grow when such a request comes. The slot is
 // free: nothing on the device reads them.
-static hx_status round_tiles(Slot& sl, const std::vector<Pending>& round, uint64_t tile) {
-  uint64_t need = 0;
-  for (const Pending& p : round) need += std::max<uint64_t>(1, (p.r.n + tile - 1) / tile);
+static hx_status round_tiles(Slot& sl, uint64_t requests, uint64_t keys, uint64_t tile) {
+  const uint64_t need = requests + keys / tile;  // a request of n keys has at most 1 + n / tile
   if (need <= sl.tile_cap) return HX_OK;
   if (need > 0xFFFFFFFFull) return HX_ERR_INVALID_ARG;
   STile *h = nullptr, *d = nullptr;
@@ -653,7 +652,7 @@ static hx_status server_step(hx_server* sv, uint32_t* launched) {
     sv->queue.pop_front();
   }
   const uint64_t tile = round_tile(keys);
-  if ((st = round_tiles(*sl, round, tile)) != HX_OK) {
+  if ((st = round_tiles(*sl, round.size(), keys, tile)) != HX_OK) {
     sv->queue.insert(sv->queue.begin(), round.begin(), round.end());  // they wait for the next step
     return st;
   }
